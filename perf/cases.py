@@ -322,7 +322,7 @@ def tolerance(case):
     if kind == "levelset":
         return {"rel": 1e-13}
     if kind == "adjoint":
-        return {"rel": 1e-9} if f64 else {"rel": 2e-3}
+        return {"rel": 1e-9} if f64 else {"rel": 2e-3, "max": 0.5}
     if kind == "bubble":
         return {"rel": 1e-10} if f64 else {"rel": 2e-6}
     return {"rel": 1e-12} if f64 else {"rel": 2e-6}
