@@ -157,7 +157,7 @@ __global__ void batch_reset_queue_kernel(int* queue) { *queue = 0; }
 template <typename T, int FLUX>
 __device__ __forceinline__ void walk_line_1d(const T* src, T* dst, int ld, int c0, int c1,
                                              T gamma, T gm1, T adi, T dtdh, int limiter,
-                                             bool muscl, bool flatten, double& ws_local,
+                                             bool muscl, bool flatten, T& ws_local,
                                              T pinf) {
   constexpr int D = 1;
   constexpr int NC = 3;
@@ -231,7 +231,7 @@ __device__ __forceinline__ void walk_line_1d(const T* src, T* dst, int ld, int c
         for (int c = 0; c < NC; ++c) r.v[c] = uo.v[c] + dtdh * (f_prev.v[c] - fx.v[c]);
 #pragma unroll
         for (int c = 0; c < NC; ++c) dst[c * ld + 4 + (j - 1)] = r.v[c];
-        ws_max(ws_local, (double)max_wavespeed_q<STIFF>(derive(r, gm1), gamma, pinf));
+        ws_max(ws_local, max_wavespeed_q<STIFF>(derive(r, gm1), gamma, pinf));
       }
       f_prev = fx;
     }
@@ -299,11 +299,11 @@ __global__ void __launch_bounds__(THREADS) batch1d_kernel(BatchArgs a, long long
       const T dtdh = (T)s_ctrl.dtdh;
       fill_ghosts_1d(cur, ld, n, reflect);
       __syncthreads();
-      double ws = 0.0;
+      T ws = T(0);
       if (c0 < n)
         walk_line_1d<T, FLUX>(cur, nxt, ld, c0, c1, gamma, gm1, adi, dtdh, a.limiter, muscl,
                               flatten, ws, pinf);
-      const double m = cta_max<THREADS / 32>(ws, s_red);
+      const double m = cta_max<THREADS / 32>((double)ws, s_red);
       if (threadIdx.x == 0) advance_control(s_ctrl, m, true);
       __syncthreads();
       T* t = cur;
@@ -349,10 +349,10 @@ __global__ void __launch_bounds__(WalkCfg<T, S>::THREADS) batch2d_kernel(BatchAr
   p.finalize = 0;
   const int warp = threadIdx.x >> 5;
   const int64_t y0 = ((int64_t)it.by * W::WARPS + warp) * pr.ry;
-  double ws_local = 0.0;
+  T ws_local = T(0);
   walk_strip_2d<T, S, FLUX>(p, dtdh, (int64_t)it.bx, y0, pr.ry, ws_local, S == 1);
   if (S == 1) {
-    const double m = cta_max<W::WARPS>(ws_local, s_red);
+    const double m = cta_max<W::WARPS>((double)ws_local, s_red);
     if (threadIdx.x == 0) {
       atomicMax(&ctrl->ws_bits, (unsigned long long)__double_as_longlong(m));
       __threadfence();

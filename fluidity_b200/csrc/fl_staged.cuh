@@ -164,7 +164,7 @@ __device__ __forceinline__ void staged_strip(const SweepParams& p, const CUtenso
                                              const CUtensorMap* tout,
                                              const StagedSmem<T, GEO, TOUT>& sm, T dtdh, T dhdt,
                                              int ab,
-                                             int s0, int ry, double& ws_local, bool want_ws,
+                                             int s0, int ry, T& ws_local, bool want_ws,
                                              uint32_t& gstage, int& fault) {
   using Cf = StagedCfg<T, GEO, TOUT>;
   constexpr int D = 2;
@@ -447,7 +447,7 @@ __device__ __forceinline__ void staged_strip(const SweepParams& p, const CUtenso
           }
         }
         if ((FAST ? S == 1 : want_ws) && owned && (FAST || ws_row_counts(p, S == 1 ? jo : ai)))
-          ws_max(ws_local, (double)max_wavespeed_q<STIFF>(derive(res, gm1), gamma, pinf));
+          ws_max(ws_local, max_wavespeed_q<STIFF>(derive(res, gm1), gamma, pinf));
       }
       f_prev = fj;
     }
@@ -507,7 +507,7 @@ __global__ void __launch_bounds__(StagedCfg<T, GEO, TOUT>::THREADS,
   }
   __syncwarp();
 
-  double ws_local = 0.0;
+  T ws_local = T(0);
   const bool want_ws = (p.ws_accum != nullptr);
   const int ry = (p.walk_ry > 0) ? p.walk_ry : Cf::RY;
   const int64_t nab = (p.n[1 - S] + 31) / 32;
@@ -542,7 +542,7 @@ __global__ void __launch_bounds__(StagedCfg<T, GEO, TOUT>::THREADS,
   }
   if (want_ws) {
     // CTA max of the lanes' wavespeeds (warp shuffles, then the CTA)
-    double v = ws_local;
+    double v = (double)ws_local;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) ws_max(v, __shfl_xor_sync(0xffffffffu, v, off));
     if (lane == 0) s_red[warp] = v;

@@ -93,7 +93,8 @@ __device__ __forceinline__ int64_t mirror_index(int64_t g, int64_t n, bool& flip
 // acc = max(acc, v), except that a NaN, once seen, stays: a non-finite
 // wavespeed anywhere must reach the step control (which stops the loop with
 // FL_ENAN), whatever the order in which cells and lanes are folded.
-__device__ __forceinline__ void ws_max(double& acc, double v) {
+template <typename T>
+__device__ __forceinline__ void ws_max(T& acc, T v) {
   if (acc == acc && !(v <= acc)) acc = v;
 }
 
@@ -330,7 +331,7 @@ sweep_kernel(SweepParams p) {
 
   // ---- stage E: conservative update, store, fused wavespeed -------------
   constexpr int FS = (S == 0) ? 1 : (S == 1 ? G::F0 : G::F0 * G::F1);
-  double ws_local = 0.0;
+  T ws_local = T(0);
   const bool want_ws = (p.ws_accum != nullptr);
   for (int o = threadIdx.x; o < G::OUT; o += NT) {
     const int t0 = o % G::T0;
@@ -348,10 +349,10 @@ sweep_kernel(SweepParams p) {
 #pragma unroll
     for (int c = 0; c < NC; ++c) out[c * pitch + gi] = r.v[c];
     if (want_ws && ws_row_counts(p, D == 1 ? g0 : (D == 2 ? g1 : g2)))
-      ws_max(ws_local, (double)max_wavespeed_q<STIFF>(derive(r, gm1), gamma, pinf));
+      ws_max(ws_local, max_wavespeed_q<STIFF>(derive(r, gm1), gamma, pinf));
   }
   if (want_ws)
-    cta_wavespeed_commit<NT>(ws_local, p.ws_accum, p.ctrl, p.finalize, true, s_red);
+    cta_wavespeed_commit<NT>((double)ws_local, p.ws_accum, p.ctrl, p.finalize, true, s_red);
 }
 
 }  // namespace fl

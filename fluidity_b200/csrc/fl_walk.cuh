@@ -75,7 +75,7 @@ __device__ __forceinline__ T shfl_dn(T v, int d) { return __shfl_down_sync(0xfff
 // from the caller.
 template <typename T, int S, int FLUX>
 __device__ __forceinline__ void walk_strip_2d(const SweepParams& p, T dtdh, int64_t bx,
-                                              int64_t y0, int ry, double& ws_local,
+                                              int64_t y0, int ry, T& ws_local,
                                               bool want_ws) {
   using W = WalkCfg<T, S>;
   constexpr int D = 2;
@@ -242,7 +242,7 @@ __device__ __forceinline__ void walk_strip_2d(const SweepParams& p, T dtdh, int6
 #pragma unroll
           for (int c = 0; c < NC; ++c) out[c * pitch + gi] = r.v[c];
           if ((FAST ? S == 1 : want_ws) && ws_row_counts(p, j))
-            ws_max(ws_local, (double)max_wavespeed_q<STIFF>(derive(r, gm1), gamma, pinf));
+            ws_max(ws_local, max_wavespeed_q<STIFF>(derive(r, gm1), gamma, pinf));
         }
       } else {
         if (j >= y0) {
@@ -259,7 +259,7 @@ __device__ __forceinline__ void walk_strip_2d(const SweepParams& p, T dtdh, int6
 #pragma unroll
             for (int c = 0; c < NC; ++c) out[c * pitch + gi] = r.v[c];
             if ((FAST ? S == 1 : want_ws) && ws_row_counts(p, j - 1))
-              ws_max(ws_local, (double)max_wavespeed_q<STIFF>(derive(r, gm1), gamma, pinf));
+              ws_max(ws_local, max_wavespeed_q<STIFF>(derive(r, gm1), gamma, pinf));
           }
           f_prev = fxy;
         }
@@ -305,7 +305,7 @@ walk_kernel_2d(SweepParams p) {
   const T dtdh = (p.ctrl != nullptr) ? (T)p.ctrl->dtdh : (T)p.dtdh;
   __shared__ double s_red[W::WARPS];
   const int warp = threadIdx.x >> 5;
-  double ws_local = 0.0;
+  T ws_local = T(0);
   const bool want_ws = (p.ws_accum != nullptr);
   // the rows to compute: [r_lo, r_hi)
   const bool win = p.row_hi > p.row_lo;
@@ -331,7 +331,7 @@ walk_kernel_2d(SweepParams p) {
     }
   }
   if (want_ws) {
-    const double m = cta_max<W::WARPS>(ws_local, s_red);
+    const double m = cta_max<W::WARPS>((double)ws_local, s_red);
     if (threadIdx.x == 0) {
       atomicMax(p.ws_accum, (unsigned long long)__double_as_longlong(m));
       if (p.finalize && p.ctrl) {

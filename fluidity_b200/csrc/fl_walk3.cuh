@@ -57,7 +57,7 @@ struct Walk3Cfg {
 template <typename T, int S, int FLUX>
 __device__ __forceinline__ void walk_strip_3d(const SweepParams& p, const T* __restrict__ xc,
                                               T dtdh, int64_t bx, int64_t y0, int ry, int64_t pl,
-                                              double& ws_local, bool want_ws) {
+                                              T& ws_local, bool want_ws) {
   using W = Walk3Cfg<T, S>;
   constexpr int D = 3;
   constexpr int NC = 5;
@@ -251,7 +251,7 @@ __device__ __forceinline__ void walk_strip_3d(const SweepParams& p, const T* __r
 #pragma unroll
         for (int c = 0; c < NC; ++c) out[c * pitch + gi] = r.v[c];
         if (FAST ? S == 2 : want_ws)
-          ws_max(ws_local, (double)max_wavespeed_q<STIFF>(derive(r, gm1), gamma, pinf));
+          ws_max(ws_local, max_wavespeed_q<STIFF>(derive(r, gm1), gamma, pinf));
       }
     } else {
       if (j >= y0) {
@@ -267,7 +267,7 @@ __device__ __forceinline__ void walk_strip_3d(const SweepParams& p, const T* __r
 #pragma unroll
           for (int c = 0; c < NC; ++c) out[c * pitch + gi] = r.v[c];
           if (FAST ? S == 2 : want_ws)
-            ws_max(ws_local, (double)max_wavespeed_q<STIFF>(derive(r, gm1), gamma, pinf));
+            ws_max(ws_local, max_wavespeed_q<STIFF>(derive(r, gm1), gamma, pinf));
         }
         f_prev = fxy;
       }
@@ -292,7 +292,7 @@ walk_kernel_3d(SweepParams p, const T* __restrict__ xc) {
   const T dtdh = (p.ctrl != nullptr) ? (T)p.ctrl->dtdh : (T)p.dtdh;
   __shared__ double s_red[W::WARPS];
   const int warp = threadIdx.x >> 5;
-  double ws_local = 0.0;
+  T ws_local = T(0);
   const bool want_ws = (p.ws_accum != nullptr);
   if (p.walk_next == nullptr) {
     const int64_t y0 = ((int64_t)blockIdx.y * W::WARPS + warp) * W::RY;
@@ -317,7 +317,7 @@ walk_kernel_3d(SweepParams p, const T* __restrict__ xc) {
     }
   }
   if (want_ws) {
-    const double m = cta_max<W::WARPS>(ws_local, s_red);
+    const double m = cta_max<W::WARPS>((double)ws_local, s_red);
     if (threadIdx.x == 0) {
       atomicMax(p.ws_accum, (unsigned long long)__double_as_longlong(m));
       if (p.finalize && p.ctrl) {
