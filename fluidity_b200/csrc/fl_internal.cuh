@@ -58,7 +58,7 @@ struct SweepParams {
   // walk_next[walk_slot] and clearing the other counter for the next sweep
   unsigned int* walk_next;
   int walk_slot;
-  int walk_ry;  // rows per strip of a dynamically scheduled 2-D walk (0: the compiled length)
+  int walk_ry;  // rows per strip of a walk, set by its launcher (strip_rows)
   // nullable: a kernel whose bounded wait on its own copies gave up writes
   // kETimeout here (and stops the loop through ctrl->done when ctrl is set)
   int* status;

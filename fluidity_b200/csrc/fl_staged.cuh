@@ -43,10 +43,6 @@
 #include "fl_sweep.cuh"
 #include "fl_tma.cuh"
 
-#ifndef FL_STAGED_RY
-#define FL_STAGED_RY 64
-#endif
-
 
 namespace fl {
 
@@ -73,7 +69,6 @@ struct StagedCfg {
   static constexpr int NS = GEO ? ((TOUT && sizeof(T) == 8) ? 7 : 8) : (sizeof(T) == 8 ? 5 : 4);
   static constexpr int WARPS = (!GEO && sizeof(T) == 8) ? 2 : 4;
   static constexpr int THREADS = 32 * WARPS;
-  static constexpr int RY = FL_STAGED_RY;
   // A tiled output collects 32 bytes along the walk per lane (one DRAM
   // sector: 4 cells in FP64, 8 in FP32) before its TMA store; 16-byte
   // stores left half-written sectors that L2 filled from DRAM, 55% more
@@ -509,7 +504,7 @@ __global__ void __launch_bounds__(StagedCfg<T, GEO, TOUT>::THREADS,
 
   T ws_local = T(0);
   const bool want_ws = (p.ws_accum != nullptr);
-  const int ry = (p.walk_ry > 0) ? p.walk_ry : Cf::RY;
+  const int ry = p.walk_ry;
   const int64_t nab = (p.n[1 - S] + 31) / 32;
   // positions along the walk to compute: a row window when the walk runs
   // along the rows (the y sweep in the grid's own layout), else all

@@ -29,9 +29,6 @@
 #include "fl_numerics.cuh"
 #include "fl_sweep.cuh"
 
-#ifndef FL_WALK_RY
-#define FL_WALK_RY 64
-#endif
 #ifndef FL_WALK_WARPS
 #define FL_WALK_WARPS 4
 #endif
@@ -54,7 +51,6 @@ template <typename T, int S>
 struct WalkCfg {
   static constexpr int HX = (S == 0) ? 4 : 3;  // halo lanes on each side
   static constexpr int OWN = 32 - 2 * HX;      // owned columns per warp
-  static constexpr int RY = FL_WALK_RY;        // rows per warp strip
   static constexpr int WARPS = FL_WALK_WARPS;  // warps per CTA (stacked strips)
   static constexpr int THREADS = 32 * WARPS;
   // resident CTAs per SM the register allocation is held to: 65536 /
@@ -310,13 +306,13 @@ walk_kernel_2d(SweepParams p) {
   // the rows to compute: [r_lo, r_hi)
   const bool win = p.row_hi > p.row_lo;
   const int64_t r_lo = win ? p.row_lo : 0, r_hi = win ? p.row_hi : p.n[1];
+  const int ry = p.walk_ry;
   if (p.walk_next == nullptr) {
-    const int64_t y0 = r_lo + ((int64_t)blockIdx.y * W::WARPS + warp) * W::RY;
+    const int64_t y0 = r_lo + ((int64_t)blockIdx.y * W::WARPS + warp) * ry;
     if (y0 < r_hi)
       walk_strip_2d<T, S, FLUX>(p, dtdh, (int64_t)blockIdx.x, y0,
-                                (int)(r_hi - y0 < W::RY ? r_hi - y0 : W::RY), ws_local, want_ws);
+                                (int)(r_hi - y0 < ry ? r_hi - y0 : ry), ws_local, want_ws);
   } else {
-    const int ry = (p.walk_ry > 0) ? p.walk_ry : W::RY;
     const int64_t ncol = (p.n[0] + W::OWN - 1) / W::OWN;
     const int64_t items = ncol * ((r_hi - r_lo + ry - 1) / ry);
     unsigned int* next = &p.walk_next[p.walk_slot];

@@ -43,7 +43,6 @@ template <typename T, int S>
 struct Walk3Cfg {
   static constexpr int HX = (S == 0) ? 4 : 3;  // halo lanes on each side
   static constexpr int OWN = 32 - 2 * HX;      // owned columns per warp
-  static constexpr int RY = FL_WALK_RY;        // rows per warp strip
   static constexpr int WARPS = FL_WALK_WARPS;  // warps per CTA (stacked strips)
   static constexpr int THREADS = 32 * WARPS;
   static constexpr int DR = (S == 2) ? 2 : 1;  // row dimension
@@ -294,16 +293,16 @@ walk_kernel_3d(SweepParams p, const T* __restrict__ xc) {
   const int warp = threadIdx.x >> 5;
   T ws_local = T(0);
   const bool want_ws = (p.ws_accum != nullptr);
+  const int ry = p.walk_ry;
   if (p.walk_next == nullptr) {
-    const int64_t y0 = ((int64_t)blockIdx.y * W::WARPS + warp) * W::RY;
+    const int64_t y0 = ((int64_t)blockIdx.y * W::WARPS + warp) * ry;
     for (int64_t pl = blockIdx.z; pl < p.n[W::DT]; pl += gridDim.z)
-      walk_strip_3d<T, S, FLUX>(p, xc, dtdh, (int64_t)blockIdx.x, y0, W::RY, pl, ws_local,
-                                want_ws);
+      walk_strip_3d<T, S, FLUX>(p, xc, dtdh, (int64_t)blockIdx.x, y0, ry, pl, ws_local, want_ws);
   } else {
     // strips taken dynamically, column group fastest, then the strip along
     // the row dimension, then the plane
     const int64_t ncol = (p.n[0] + W::OWN - 1) / W::OWN;
-    const int64_t nrow = (p.n[W::DR] + W::RY - 1) / W::RY;
+    const int64_t nrow = (p.n[W::DR] + ry - 1) / ry;
     const int64_t items = ncol * nrow * p.n[W::DT];
     unsigned int* next = &p.walk_next[p.walk_slot];
     for (;;) {
@@ -312,7 +311,7 @@ walk_kernel_3d(SweepParams p, const T* __restrict__ xc) {
       item = __shfl_sync(0xffffffffu, item, 0);
       if ((int64_t)item >= items) break;
       const int64_t cr = (int64_t)item % (ncol * nrow);
-      walk_strip_3d<T, S, FLUX>(p, xc, dtdh, cr % ncol, (cr / ncol) * W::RY, W::RY,
+      walk_strip_3d<T, S, FLUX>(p, xc, dtdh, cr % ncol, (cr / ncol) * ry, ry,
                                 (int64_t)item / (ncol * nrow), ws_local, want_ws);
     }
   }
@@ -341,7 +340,7 @@ walk_kernel_3d(SweepParams p, const T* __restrict__ xc) {
 // DT are mirror ghosts with the reflective flip.
 template <typename T, int S>
 __global__ void __launch_bounds__(Walk3Cfg<T, S>::THREADS)
-chi_dim_kernel(SweepParams p, T* __restrict__ xc) {
+chi_dim_kernel(SweepParams p, T* __restrict__ xc, int ry) {
   using W = Walk3Cfg<T, S>;
   constexpr int D = 3;
   constexpr int NC = 5;
@@ -357,9 +356,9 @@ chi_dim_kernel(SweepParams p, T* __restrict__ xc) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t x = (int64_t)blockIdx.x * 32 + lane;
   const int64_t gx = x < n0 ? x : n0 - 1;
-  const int64_t j0 = ((int64_t)blockIdx.y * W::WARPS + warp) * W::RY;
+  const int64_t j0 = ((int64_t)blockIdx.y * W::WARPS + warp) * ry;
   if (j0 >= nt) return;
-  const int64_t j_end = (j0 + W::RY < nt) ? j0 + W::RY : nt;
+  const int64_t j_end = (j0 + ry < nt) ? j0 + ry : nt;
   for (int64_t pl = blockIdx.z; pl < p.n[DR]; pl += gridDim.z) {
     const int64_t base = pl * ps;
     T P[5], V[5], CH[3];

@@ -236,6 +236,24 @@ def test_3d_walk_shapes(cuda, oracle, shape, dtype):
             assert abs(got_ws - ref_ws) <= (1e-14 if dtype == "f64" else 1e-6) * ref_ws
 
 
+@pytest.mark.parametrize("shape", [(24, 4), (25, 37), (60, 900), (700, 61), (64, 64), (9, 8, 150),
+                                   (130, 40, 6)],
+                         ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+def test_strip_lengths_match_oracle(cuda, oracle, shape, dtype):
+    """Grids whose walks take strips of 4 to 64 rows (a launch picks the
+    length by the rows, the column groups and the resident warps), with a
+    remainder strip or a single one: each sweep against the oracle."""
+    u = oracle.prim_to_cons(random_prim(shape, 5, smooth=True, mild=True), GAMMA,
+                            dtype=NPDT[dtype])
+    for dim in range(len(shape)):
+        want = oracle.sweep(shape, dim, u, NPDT[dtype](GAMMA), NPDT[dtype](0.05))
+        got, ws = gpu_sweep(shape, dim, u, 0.05, dtype=dtype, want_ws=True)
+        assert err(got, want, dtype) < TOL[dtype], dim
+        top = oracle.max_wavespeed(shape, want, NPDT[dtype](GAMMA))
+        assert abs(ws - top) < 10 * TOL[dtype] * top, dim
+
+
 @pytest.mark.parametrize("shape", [(100001,), (317, 211), (37, 29, 23)],
                          ids=lambda s: "x".join(map(str, s)))
 @pytest.mark.parametrize("where", ["first", "middle", "last"])
