@@ -756,6 +756,18 @@ int fl_sim_steps(fl_sim* sim, int64_t nsteps, void* stream) {
       return kOk;
     }
   }
+  // 1-D: all the steps in one launch.  A row window for the wavespeed keeps
+  // one launch per step.
+  const int ranks = (D == 1 && !(sim->own_hi > sim->own_lo))
+                        ? line_loop_ranks(sim->grid.n[0], sim->pol.f32)
+                        : 0;
+  if (ranks > 0 && nsteps > 0) {
+    const cudaError_t e = launch_line_loop(p, sim->pol.f32, sim->pol.flux, sim->a, sim->b, nsteps,
+                                           ranks, st);
+    if (e != cudaSuccess) return cuda_fail(e, "fl_sim_steps");
+    sim->enqueued += nsteps;
+    return kOk;
+  }
   for (int64_t k = 0; k < nsteps; ++k) {
     // input of this step: for even D the state returns to buffer a every
     // step; for odd D it alternates a, b, a, ...
@@ -946,15 +958,18 @@ int fl_simulate(fl_sim* sim, void* a, void* b, double cfl, double res, double si
   if (rc) return rc;
   int done = 0;
   int64_t it = 0;
+  // Each chunk ends with a wait for the stream (about 20 us), so the first is
+  // enqueued without one (the steps of a run that is over do nothing), and
+  // the 1-D loop, which stops by itself inside its launch, takes long ones.
+  const bool line = sim->grid.dims == 1 && line_loop_ranks(sim->grid.n[0], sim->pol.f32) > 0;
+  const int64_t most = line ? 4096 : 64;
   while (true) {
+    const int64_t left = max_iters - sim->enqueued;
+    const int64_t chunk = left < most ? left : most;
+    if (chunk > 0 && (rc = fl_sim_steps(sim, chunk, stream))) return rc;
     rc = fl_sim_status(sim, stream, &it, run_time, &done, result);
     if (rc) return rc;
-    if (done) break;
-    const int64_t left = max_iters - sim->enqueued;
-    const int64_t chunk = left < 64 ? left : 64;
-    if (chunk <= 0) break;
-    rc = fl_sim_steps(sim, chunk, stream);
-    if (rc) return rc;
+    if (done || chunk <= 0) break;
   }
   if (iters) *iters = it;
   return kOk;

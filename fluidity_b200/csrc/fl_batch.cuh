@@ -70,30 +70,6 @@ constexpr int batch1d_max() {
   return (int)((220 * 1024) / (2 * 3 * sizeof(T))) - 8;
 }
 
-// Advance one problem's control after a step given the step's max wavespeed
-// (Parameters::update_simulation_info / update_time_delta /
-// continue_simulation, simulator/parameters.hpp:60-77).
-__device__ __forceinline__ void advance_control(StepControl& c, double ws, bool advance) {
-  if (advance) {
-    if (c.is_f32) c.run_time = (double)((float)c.run_time + (float)c.dt);
-    else c.run_time = c.run_time + c.dt;
-    c.iters += 1;
-  }
-  if (c.is_f32) {
-    c.dt = (double)(float)((double)(float)c.cfl * c.res / (double)(float)ws);
-    c.dtdh = (double)(float)(c.dt / c.res);
-  } else {
-    c.dt = c.cfl * c.res / ws;
-    c.dtdh = c.dt / c.res;
-  }
-  bool cont = (c.run_time < c.sim_time) && (c.iters < c.max_iters);
-  if (!(ws > 0.0) || !(ws <= DBL_MAX)) {
-    c.status = kENan;
-    cont = false;
-  }
-  c.done = cont ? 0 : 1;
-}
-
 // ---- initial wavespeed of every problem (one CTA per problem) -------------
 
 template <typename T>

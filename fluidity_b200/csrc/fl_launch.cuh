@@ -19,4 +19,12 @@ cudaError_t launch_sweep_f32(const SweepParams& p, int dims, int dim, int flux,
 bool loop_transposes_f64(const SweepParams& p, int flux);
 bool loop_transposes_f32(const SweepParams& p, int flux);
 
+// The 1-D loop in one launch (fl_line.cu): up to nsteps steps of the control
+// block p.ctrl on the buffers a and b, by a cluster of `ranks` CTAs.
+// line_loop_ranks gives that count for a grid of n cells, or 0 where one
+// launch per step is the faster form.
+int line_loop_ranks(int64_t n, bool f32);
+cudaError_t launch_line_loop(const SweepParams& p, bool f32, int flux, void* a, void* b,
+                             int64_t nsteps, int ranks, cudaStream_t stream);
+
 }  // namespace fl

@@ -1,0 +1,327 @@
+// fl_line.cu -- the 1-D time loop, whole steps in one launch.
+//
+// The loop of SimulatorImpl::simulate (simulator/simulator_impl.hpp:223-258)
+// on a 1-D grid: per step one sweep (solver/split_solver.hpp:138-162) with
+// the arithmetic of sweep_kernel (fl_sweep.cuh), the max wavespeed of the new
+// state and the next time step (simulator/parameters.hpp:60-77).
+//
+// A tube of a few hundred to some thousand cells is bound by latency: one
+// launch per step took 8.8 us a step at 400 cells in FP64.  Here one cluster of
+// CTAs keeps the state in shared memory for all the steps of a launch:
+//   * a warp takes 32 consecutive cells, of which its middle 24 are its own
+//     (the stencil reaches 4 cells); neighbours' derived values come from warp
+//     shuffles, so a step needs no barrier inside it;
+//   * owned cells go to the other of two shared buffers, and the four next to
+//     an end of the CTA's range also to the neighbour CTA's halo
+//     (distributed shared memory) or, at an end of the domain, to the mirror
+//     ghosts;
+//   * each warp's max wavespeed goes to every CTA of the cluster, then one
+//     barrier (of the CTA, or of the cluster) ends the step, and every warp
+//     folds the maxima and takes the next time step on its own.
+// A step takes 2.3 us at 400 cells in FP64 and 1.7 in FP32, the latency of
+// one cell's chain of dependent operations.
+// Waits are the hardware's barriers only, and every thread leaves the loop at
+// the same step: all of them fold the same values.
+#include <cooperative_groups.h>
+#include <cuda_runtime.h>
+
+#include <cfloat>
+#include <cstdlib>
+#include <cstring>
+#include <type_traits>
+
+#include "fl_internal.cuh"
+#include "fl_launch.cuh"
+#include "fl_numerics.cuh"
+#include "fl_sweep.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace fl {
+namespace {
+
+constexpr int kOwn = 24;       // cells a warp updates
+constexpr int kMaxWarps = 20;  // 640 threads: up to 96 registers each
+constexpr int kMaxCluster = 8;
+
+// Largest value of the warp as a max of the bit patterns: a wavespeed is
+// non-negative or NaN, and a NaN's bits exceed every number's.
+__device__ __forceinline__ float warp_max_bits(float v) {
+  return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
+}
+__device__ __forceinline__ double warp_max_bits(double v) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  return __hiloint2double((int)mh, (int)ml);
+}
+
+template <typename T>
+__device__ __forceinline__ T up(T v, int d) { return __shfl_up_sync(0xffffffffu, v, d); }
+template <typename T>
+__device__ __forceinline__ T dn(T v, int d) { return __shfl_down_sync(0xffffffffu, v, d); }
+
+// New state of this lane's cell (valid on lanes 4..27), x its index in the
+// planes of `src` (plane stride ld).
+template <typename T, int FLUX, int LIM, bool MUSCL, bool FLAT>
+__device__ __forceinline__ Cons<T, 1> line_cell(const T* src, int ld, int x, T gamma, T gm1, T adi,
+                                                T dtdh, T dhdt, T pinf) {
+  constexpr int NC = 3;
+  Cons<T, 1> u, er, el;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) u.v[c] = src[c * ld + x];
+  if constexpr (MUSCL) {
+    T ch = T(0.5);
+    if constexpr (FLAT) {
+      const Derived<T, 1> q = derive(u, gm1);
+      const T pr = dn(q.p, 1), pl = up(q.p, 1);
+      const T base = (T)chi_base<T>(pr, pl, dn(q.p, 2), up(q.p, 2), up(q.v[0], 1), dn(q.v[0], 1));
+      const T br = dn(base, 1), bl = up(base, 1);
+      const T dx = pr - pl;
+      ch *= std_min(base, dx > T(0) ? br : (dx < T(0) ? bl : base));
+    }
+    const int xm = x > 0 ? x - 1 : 0, xp = x + 1 < ld ? x + 1 : x;  // edge lanes: unused
+    Cons<T, 1> a, b, fa, fb;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const T d = ch * limited_slope<T>(LIM, u.v[c] - src[c * ld + xm], src[c * ld + xp] - u.v[c]);
+      a.v[c] = u.v[c] - d;
+      b.v[c] = u.v[c] + d;
+    }
+    flux_q(a, derive(a, gm1), 0, fa);
+    flux_q(b, derive(b, gm1), 0, fb);
+    const T hd = T(0.5) * dtdh;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const T df = fa.v[c] - fb.v[c];
+      er.v[c] = b.v[c] + hd * df;
+      el.v[c] = a.v[c] + hd * df;
+    }
+  } else {
+    er = u;
+    el = u;
+  }
+  Cons<T, 1> ul, f;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) ul.v[c] = up(er.v[c], 1);
+  riemann_qh<FLUX>(ul, derive(ul, gm1), el, derive(el, gm1), 0, gamma, gm1, adi, dtdh, dhdt, f,
+                   pinf);
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const T fr = dn(f.v[c], 1);
+    u.v[c] = u.v[c] + dtdh * (f.v[c] - fr);
+  }
+  return u;
+}
+
+template <typename T, int FLUX>
+__global__ void __launch_bounds__(32 * kMaxWarps, 1)
+    line_loop_kernel(SweepParams p, T* bufa, T* bufb, long long nsteps, int per) {
+  constexpr int NC = 3;
+  constexpr bool STIFF = (FLUX & kStiffEos) != 0;
+  extern __shared__ __align__(16) unsigned char line_smem[];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int ranks = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // two state buffers of 3 planes with 4 halo cells per side, then the
+  // wavespeed maxima of every warp of the cluster, for odd and even steps
+  const int ld = per + 8;
+  T* const s0 = reinterpret_cast<T*>(line_smem);
+  T* const sws = s0 + 2 * NC * ld;
+  const int nws = ranks * warps;
+
+  const StepControl c0 = *p.ctrl;
+  if (c0.done) return;  // every thread of the cluster alike
+  const int n = (int)p.n[0];
+  const int lo = rank * per;                          // first cell of this CTA
+  const int cells = (n - lo < per) ? n - lo : per;    // its count
+  const T* in = (c0.iters & 1) ? bufb : bufa;
+  for (int i = threadIdx.x; i < cells + 8; i += blockDim.x) {
+    bool f = false;
+    const int g = (int)mirror_index((int64_t)lo + i - 4, (int64_t)n, f);
+    Cons<T, 1> u;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) u.v[c] = in[c * p.pitch + g];
+    if (f && (p.reflect & 1u)) u.v[2] = (-(u.v[2] / u.v[0])) * u.v[0];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) s0[c * ld + i] = u.v[c];
+  }
+  // neighbours' shared memory is written to from the first step on
+  if (ranks > 1) cluster.sync();
+  else __syncthreads();
+
+  const T gamma = (T)p.gamma, gm1 = gamma - T(1), adi = (gamma + T(1)) / (T(2) * gamma);
+  const T pinf = (T)p.pinf;
+  const bool first = rank == 0, last = rank == ranks - 1;
+  T* const left = first ? nullptr : cluster.map_shared_rank(s0, rank - 1);
+  T* const right = last ? nullptr : cluster.map_shared_rank(s0, rank + 1);
+  const bool refl = (p.reflect & 1u) != 0;
+
+  StepControl c = c0;
+  int cur = 0;
+  long long step = 0;
+  auto loop = [&](auto lim, auto muscl, auto flat) {
+    for (; step < nsteps && !c.done; ++step) {
+      const T dtdh = (T)c.dtdh;
+      const T dhdt = T(1.0) / dtdh;
+      const T* src = s0 + cur * NC * ld;
+      const int off = (1 - cur) * NC * ld;  // the other buffer, here and in the neighbours
+      T ws = T(0);
+      for (int x0 = warp * kOwn; x0 < cells; x0 += warps * kOwn) {
+        const int x = x0 - 4 + lane;  // cell of this CTA; halo index x + 4
+        const int xi = x + 4 < cells + 8 ? x + 4 : cells + 7;
+        const Cons<T, 1> r =
+            line_cell<T, FLUX, decltype(lim)::value, decltype(muscl)::value,
+                      decltype(flat)::value>(src, ld, xi, gamma, gm1, adi, dtdh, dhdt, pinf);
+        if (lane >= 4 && lane < 4 + kOwn && x < cells) {
+          ws_max(ws, max_wavespeed_q<STIFF>(derive(r, gm1), gamma, pinf));
+          // where else the cell goes: a neighbour's halo or a mirror ghost
+          T* other = nullptr;
+          T* other2 = nullptr;
+          T gm = r.v[2];
+          if (x < 4) {
+            const int nl = per;  // every CTA but the last holds `per` cells
+            other = first ? s0 + off + 3 - x : left + off + 4 + nl + x;
+          }
+          if (x >= cells - 4)
+            other2 = last ? s0 + off + 4 + 2 * cells - 1 - x : right + off + x - (cells - 4);
+          if (refl) gm = (-(r.v[2] / r.v[0])) * r.v[0];
+          T* d = s0 + off + 4 + x;
+#pragma unroll
+          for (int k = 0; k < NC; ++k) d[k * ld] = r.v[k];
+          if (other != nullptr) {
+#pragma unroll
+            for (int k = 0; k < NC; ++k) other[k * ld] = (k == 2 && first) ? gm : r.v[k];
+          }
+          if (other2 != nullptr) {
+#pragma unroll
+            for (int k = 0; k < NC; ++k) other2[k * ld] = (k == 2 && last) ? gm : r.v[k];
+          }
+        }
+      }
+      ws = warp_max_bits(ws);
+      T* const wsp = sws + (step & 1) * nws;
+      if (lane < ranks) {
+        T* dst = (lane == rank) ? wsp : cluster.map_shared_rank(wsp, lane);
+        dst[rank * warps + warp] = ws;
+      }
+      if (ranks > 1) cluster.sync();
+      else __syncthreads();
+      T m = T(0);
+      for (int i = lane; i < nws; i += 32) ws_max(m, wsp[i]);
+      advance_control(c, (double)warp_max_bits(m), true);
+      cur ^= 1;
+    }
+  };
+  using VL = std::integral_constant<int, kVanLeer>;
+  using SB = std::integral_constant<int, kSuperbee>;
+  if (p.basic)
+    loop(VL{}, std::false_type{}, std::false_type{});
+  else if (p.limiter == kSuperbee && p.flatten)
+    loop(SB{}, std::true_type{}, std::true_type{});
+  else if (p.limiter == kSuperbee)
+    loop(SB{}, std::true_type{}, std::false_type{});
+  else if (p.flatten)
+    loop(VL{}, std::true_type{}, std::true_type{});
+  else
+    loop(VL{}, std::true_type{}, std::false_type{});
+
+  // the result alternates between the buffers, as with one launch per step
+  T* out = (c.iters & 1) ? bufb : bufa;
+  const T* src = s0 + cur * NC * ld;
+  for (int i = threadIdx.x; i < cells; i += blockDim.x)
+#pragma unroll
+    for (int k = 0; k < NC; ++k) out[k * p.pitch + lo + i] = src[k * ld + 4 + i];
+  if (first && threadIdx.x == 0) {
+    p.ctrl->dt = c.dt;
+    p.ctrl->dtdh = c.dtdh;
+    p.ctrl->run_time = c.run_time;
+    p.ctrl->iters = c.iters;
+    p.ctrl->status = c.status;
+    p.ctrl->done = c.done;
+  }
+}
+
+template <typename T, int FLUX>
+cudaError_t launch_line(const SweepParams& p, void* a, void* b, int64_t nsteps, int ranks,
+                        cudaStream_t st) {
+  const int n = (int)p.n[0];
+  const int per = (n + ranks - 1) / ranks;
+  const int items = (per + kOwn - 1) / kOwn;
+  // the warps share the items evenly
+  const int rounds = (items + kMaxWarps - 1) / kMaxWarps;
+  const int warps = (items + rounds - 1) / rounds;
+  const size_t smem = ((size_t)2 * 3 * (per + 8) + 2 * (size_t)ranks * warps) * sizeof(T);
+  auto kernel = line_loop_kernel<T, FLUX>;
+  static bool configured[64] = {false};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev >= 64) return cudaErrorInvalidDevice;
+  if (!configured[dev]) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (e != cudaSuccess) return e;
+    configured[dev] = true;
+  }
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)ranks);
+  cfg.blockDim = dim3((unsigned)(32 * warps));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)ranks;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  e = cudaLaunchKernelEx(&cfg, kernel, p, static_cast<T*>(a), static_cast<T*>(b),
+                         (long long)nsteps, per);
+  if (e != cudaSuccess) return e;
+  return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t launch_line_t(const SweepParams& p, int flux, void* a, void* b, int64_t nsteps,
+                          int ranks, cudaStream_t st) {
+  switch (flux | (p.pinf != 0.0 ? kStiffEos : 0)) {
+    case kHllc: return launch_line<T, kHllc>(p, a, b, nsteps, ranks, st);
+    case kForce: return launch_line<T, kForce>(p, a, b, nsteps, ranks, st);
+    case kLaxFriedrichs: return launch_line<T, kLaxFriedrichs>(p, a, b, nsteps, ranks, st);
+    case kRichtmyer: return launch_line<T, kRichtmyer>(p, a, b, nsteps, ranks, st);
+    case kHllc | kStiffEos: return launch_line<T, kHllc | kStiffEos>(p, a, b, nsteps, ranks, st);
+    case kForce | kStiffEos: return launch_line<T, kForce | kStiffEos>(p, a, b, nsteps, ranks, st);
+    case kLaxFriedrichs | kStiffEos:
+      return launch_line<T, kLaxFriedrichs | kStiffEos>(p, a, b, nsteps, ranks, st);
+    case kRichtmyer | kStiffEos:
+      return launch_line<T, kRichtmyer | kStiffEos>(p, a, b, nsteps, ranks, st);
+  }
+  return cudaErrorInvalidValue;
+}
+
+}  // namespace
+
+// CTAs of the cluster for n cells, or 0: one launch per step instead.  Steps
+// of a 200-step HLLC run, us, with 1 / 2 / 4 / 8 CTAs (8.8 with one launch per
+// step at any of these sizes):
+//   FP64  100 cells 2.7 2.8 2.8 2.8   400 cells 3.3 3.0 2.8 2.7
+//         1500 cells 7.4 4.6 3.3 2.9  6000 cells - - 7.6 4.7  12000 - - - 7.7
+//   FP32  100 cells 1.9 2.1 2.1 2.1   400 cells 2.3 2.3 2.1 2.1
+//         1500 cells 4.6 3.1 2.4 2.1  12000 cells - - - 4.9
+// so the cluster's barrier costs about as much as the CTA's, and eight CTAs
+// win from a few hundred cells on, until they take as long as a launch.
+int line_loop_ranks(int64_t n, bool f32) {
+  static const char* mode = std::getenv("FLUIDITY_B200_SWEEP");
+  if (mode != nullptr && std::strcmp(mode, "tile") == 0) return 0;
+  if (n > kMaxCluster * (f32 ? 3072 : 1536)) return 0;
+  return n <= 240 ? 1 : kMaxCluster;
+}
+
+cudaError_t launch_line_loop(const SweepParams& p, bool f32, int flux, void* a, void* b,
+                             int64_t nsteps, int ranks, cudaStream_t stream) {
+  return f32 ? launch_line_t<float>(p, flux, a, b, nsteps, ranks, stream)
+             : launch_line_t<double>(p, flux, a, b, nsteps, ranks, stream);
+}
+
+}  // namespace fl

@@ -613,3 +613,62 @@ def test_workspace_3d_walk_and_tile_match_oracle(cuda, oracle, dtype):
             s.sweep(a, b, dim, float(dtdh))
             torch.cuda.synchronize()
             assert err(b.cpu().numpy(), ref, dtype) < TOL[dtype], (workspace, dim)
+
+
+@pytest.mark.parametrize("n", [4, 7, 24, 25, 240, 241, 480, 1531, 12288])
+@pytest.mark.parametrize("dtype,flux,limiter,recon,reflect,flatten", [
+    ("f64", "hllc", "vanleer", "muscl", 0, True), ("f32", "force", "superbee", "muscl", 1, True),
+    ("f64", "richtmyer", "vanleer", "basic", 1, True), ("f32", "hllc", "vanleer", "muscl", 1, False)])
+def test_line_loop_equals_step_launches(cuda, n, dtype, flux, limiter, recon, reflect, flatten):
+    """The 1-D loop in one launch (one CTA up to 240 cells, a cluster of eight
+    beyond) against one sweep launch per step (fl_sim_sweep), with an odd
+    number of steps split over two calls: state, buffer, time and count.  Both
+    round the same expressions; the compiler may contract them differently."""
+    import torch
+    from fluidity_b200 import capi
+    from fluidity_b200.solver import Simulation, SplitSolver, _stream_ptr
+    s = SplitSolver((n,), dtype=dtype, flux=flux, limiter=limiter, recon=recon, gamma=GAMMA,
+                    boundary_mask=reflect, flatten=flatten)
+    u = to_dev(random_prim((n,), n, smooth=True, mild=True), dtype)
+    u[1] = u[1] / (GAMMA - 1) + 0.5 * u[0] * u[2] * u[2]
+    u[2] = u[0] * u[2]
+    runs = []
+    for line in (True, False):
+        sim, a, b = Simulation(s), u.clone(), torch.zeros_like(u)
+        sim.begin(a, b, 0.5, 1.0 / n, 1e30, 9)
+        for k in (4, 3):
+            if line:
+                sim.steps(k)
+            else:
+                for _ in range(k):
+                    capi.check(s.lib.fl_sim_sweep(sim.handle, 0, _stream_ptr()), s.lib)
+        it, t, done, res = sim.status()
+        runs.append((it, t, done, res is b, res.cpu().numpy()))
+    x, y = runs
+    assert x[0] == y[0] == 7 and x[2] == y[2] and x[3] and y[3]
+    assert abs(x[1] - y[1]) <= (1e-13 if dtype == "f64" else 1e-5) * y[1]
+    assert err(x[4], y[4], dtype) < TOL[dtype]
+
+
+def test_line_loop_stops_where_step_launches_do(cuda):
+    """A run that reaches its end time inside a launch, a run that blows up
+    there, and steps enqueued after the end."""
+    import torch
+    from fluidity_b200 import capi
+    from fluidity_b200.solver import Simulation, SplitSolver
+    s = SplitSolver((300,), dtype="f64", gamma=GAMMA)
+    u = s.fill_riemann([[1.0, 1.0, 0.0], [0.125, 0.1, 0.0]])
+    sim, a, b = Simulation(s), u.clone(), torch.empty_like(u)
+    sim.begin(a, b, 0.8, 1.0 / 300, 0.05, 10 ** 6)
+    sim.steps(1000)
+    it, t, done, res = sim.status()
+    keep = res.clone()
+    sim.steps(3)
+    assert sim.status()[:3] == (it, t, True) and done and 0.05 <= t < 0.06
+    assert torch.equal(sim.status()[3], keep)
+    u[1, 150] = float("nan")
+    sim.begin(u.clone(), b, 0.8, 1.0 / 300, 0.05, 10 ** 6)
+    sim.steps(5)
+    with pytest.raises(capi.FlError):
+        sim.status()
+    assert sim.status(allow_nan=True)[0] == 0
