@@ -18,12 +18,16 @@
 //     TMA store writes back when its columns are complete.
 // Each warp owns a ring of stages in shared memory, each with an mbarrier;
 // lane 0 keeps the ring filled ahead of the walk.  The stencil along the
-// sweep reads the ring (own lane only, no exchange).  The stencil across the
-// sweep -- the flattening coefficient's pressure and velocity reach of 3 --
-// goes through two small per-warp exchange rows (pressure and velocity);
-// the 6 across-halo cells (3 on each side of the warp) are derived in one
-// extra pass of all lanes, of which lanes 0-5 keep theirs (no divergent
-// region), and each lane computes the flattening base of the neighbour its
+// sweep reads the ring (own lane only, no exchange).  The flattening
+// coefficient is 1 except at strong shocks: an integer screen of the
+// pressures (press_key, may_flatten in fl_numerics.cuh) votes per position
+// whether any lane can be flattened, and the pressures of the warp's edges
+// are derived for four positions at once, one per lane.  Where the vote
+// passes, the stencil across the sweep -- the coefficient's pressure and
+// velocity reach of 3 -- goes through two small per-warp exchange rows
+// (pressure and velocity); the 6 across-halo cells (3 on each side of the
+// warp) are derived in one extra pass of all lanes, of which lanes 0-5 keep
+// theirs, and each lane computes the flattening base of the neighbour its
 // pressure rises towards itself, from those rows.
 // The reference's halo of 4 along the sweep costs 7 extra derivations per
 // strip of 64 and one extra evolve and Riemann solve at its start.
@@ -200,6 +204,11 @@ __device__ __forceinline__ void staged_strip(const SweepParams& p, const CUtenso
   hoff = hoff < 0 ? 0 : (hoff >= Cf::BW ? Cf::BW - 1 : hoff);
   const bool flip_h = fh && flip_a_on;
   const int hx = (lane < 3) ? Cf::AOFF - 3 + lane : Cf::AOFF + 29 + lane;
+  // the cell this lane screens for the warp's edges
+  const int ei = a0 - 2 + (lane & 3) + ((lane & 4) << 3);
+  bool fe = false;
+  int eoff = (int)mirror_index(ei, na, fe) - (a0 - Cf::AOFF);
+  eoff = eoff < 0 ? 0 : (eoff >= Cf::BW ? Cf::BW - 1 : eoff);
 
   const int s_end = (s0 + ry < nl) ? s0 + ry : nl;
   const int k_first = s0 - 4;
@@ -255,16 +264,19 @@ __device__ __forceinline__ void staged_strip(const SweepParams& p, const CUtenso
   auto ghost_l = [&](int k) { return flip_l_on && (unsigned)k >= (unsigned)nl; };
 
   // windows along the sweep: index 4 = newest position k, k - i at 4 - i
-  T P[5], VL[5];
+  T P[5];
   T CHA[3];   // flattening base along the sweep at k-4, k-3, k-2
-  T CX[4];    // across part of chi at k-3 .. k
   Cons<T, D> er_prev, f_prev;
 #pragma unroll
-  for (int i = 0; i < 5; ++i) { P[i] = T(0); VL[i] = T(0); }
+  for (int i = 0; i < 5; ++i) P[i] = T(0);
 #pragma unroll
   for (int i = 0; i < 3; ++i) CHA[i] = T(1);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) CX[i] = T(1);
+  // the screen: keys of positions k-1 and k-2, and per position (bit i: k-i)
+  // whether some lane may be flattened along the sweep at the position before
+  // it or across the sweep at it; halo: the same across the sweep for the
+  // bases at the warp's two edges, for the next four evolve positions
+  uint32_t key1 = 0u, key2 = 0u, hist = 0u;
+  bool halo = false;
 
   T* const out = static_cast<T*>(p.out);
   const int64_t pitch = p.pitch;
@@ -311,50 +323,38 @@ __device__ __forceinline__ void staged_strip(const SweepParams& p, const CUtenso
     const Cons<T, D> u = load(stk, qk, aoff, glk, RF && flip_a);
     const Derived<T, D> q = derive(u, gm1);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      P[i] = P[i + 1];
-      VL[i] = VL[i + 1];
-    }
+    for (int i = 0; i < 4; ++i) P[i] = P[i + 1];
     P[4] = q.p;
-    VL[4] = q.v[S];
-    T cx = T(1);
     if (flat) {
-      sm.xp[own] = q.p;
-      sm.xv[own] = q.v[1 - S];
-      {
-        // every lane derives a halo cell (lanes 0-5 keep theirs): no
-        // divergent region between the own and the halo derivations
-        const Cons<T, D> uh = load(stk, qk, hoff, glk, RF && flip_h);
-        const Derived<T, D> qh = derive(uh, gm1);
-        if (lane < 6) {
-          sm.xp[hx] = qh.p;
-          sm.xv[hx] = qh.v[1 - S];
-        }
+      const uint32_t key = press_key(q.p);
+      const bool steep = may_flatten<T>(key, key2) |
+                         may_flatten<T>(key, __shfl_up_sync(0xffffffffu, key, 2));
+      hist = 2u * hist + (__any_sync(0xffffffffu, steep) ? 1u : 0u);
+      key2 = key1;
+      key1 = key;
+      if (r >= 6 && (r & 3) == 2) {
+        // the edges' bases, four rows at once: lane 8 i + c derives cell c
+        // (-2, -1, 0, 1, 30, 31, 32, 33 across) of position k - 3 + i
+        int qh;
+        const T* sth = stage_back(r, 3 - (lane >> 3), qh);
+        const uint32_t kh = press_key(derive(load(sth, qh, eoff, false, false), gm1).p);
+        const uint32_t kn = __shfl_down_sync(0xffffffffu, kh, 2);
+        const bool edge = (lane & 2) == 0 && may_flatten<T>(kh, kn);
+        halo = __any_sync(0xffffffffu, edge);
       }
-      __syncwarp();
-      const T pr1 = sm.xp[own + 1], pl1 = sm.xp[own - 1];
-      const T pr2 = sm.xp[own + 2], pl2 = sm.xp[own - 2];
-      const T vr1 = sm.xv[own + 1], vl1 = sm.xv[own - 1];
-      const T dx = pr1 - pl1;
-      const int sx = (T(0) < dx) - (dx < T(0));
-      // the two values the neighbour the pressure rises towards needs beyond
-      // this lane's own reach
-      const T p3 = sm.xp[own + 3 * sx], v2 = sm.xv[own + 2 * sx];
-      __syncwarp();  // every lane has read the exchange rows
-      const T chx = (T)chi_base<T>(pr1, pl1, pr2, pl2, vl1, vr1);
-      const T qp = q.p, qv = q.v[1 - S];
-      const bool upw = sx > 0;
-      const T cn = (T)chi_base<T>(upw ? pr2 : qp, upw ? qp : pl2, upw ? p3 : pr1, upw ? pl1 : p3,
-                                  upw ? qv : v2, upw ? v2 : qv);
-      cx = std_min(chx, sx != 0 ? cn : chx);
+      // ---- flattening base along the sweep of position k - 2 -------------
+      // (bit 4: the base that leaves the window)
+      if (hist & 0x1eu) {
+        CHA[0] = CHA[1];
+        CHA[1] = CHA[2];
+        int q3, q1;
+        const T* s3 = stage_back(r, r < 3 ? 0 : 3, q3);
+        const T* s1 = stage_back(r, r < 1 ? 0 : 1, q1);
+        const T v3 = derive(load(s3, q3, aoff, RF && ghost_l(k - 3), RF && flip_a), gm1).v[S];
+        const T v1 = derive(load(s1, q1, aoff, RF && ghost_l(k - 1), RF && flip_a), gm1).v[S];
+        CHA[2] = (T)chi_base<T>(P[3], P[1], P[4], P[0], v3, v1);
+      }
     }
-#pragma unroll
-    for (int i = 0; i < 3; ++i) CX[i] = CX[i + 1];
-    CX[3] = cx;
-    // ---- flattening base along the sweep of position k - 2 ---------------
-    CHA[0] = CHA[1];
-    CHA[1] = CHA[2];
-    if (flat) CHA[2] = (T)chi_base<T>(P[3], P[1], P[4], P[0], VL[1], VL[3]);
 
     const int j = k - 3;  // evolve position
     if (j < s0 - 1) continue;
@@ -372,14 +372,42 @@ __device__ __forceinline__ void staged_strip(const SweepParams& p, const CUtenso
       int qp;
       const T* stp = stage_back(r, 2, qp);
       const Cons<T, D> up = load(stp, qp, aoff, RF && ghost_l(j + 1), RF && flip_a);
-      T chi_v = T(1);
-      if (flat) {
+      T ch = T(0.5);
+      if (flat && ((hist & 0xeu) != 0u || halo)) {
+        // ---- flattening across the sweep of (lane, j) ---------------------
+        const T qp = P[1];
+        const T qv = derive(uj, gm1).v[1 - S];
+        sm.xp[own] = qp;
+        sm.xv[own] = qv;
+        {
+          // every lane derives a halo cell (lanes 0-5 keep theirs)
+          const Cons<T, D> uh = load(stj, qj, hoff, RF && ghost_l(j), RF && flip_h);
+          const Derived<T, D> qh = derive(uh, gm1);
+          if (lane < 6) {
+            sm.xp[hx] = qh.p;
+            sm.xv[hx] = qh.v[1 - S];
+          }
+        }
+        __syncwarp();
+        const T pr1 = sm.xp[own + 1], pl1 = sm.xp[own - 1];
+        const T pr2 = sm.xp[own + 2], pl2 = sm.xp[own - 2];
+        const T vr1 = sm.xv[own + 1], vl1 = sm.xv[own - 1];
+        const T dx = pr1 - pl1;
+        const int sx = (T(0) < dx) - (dx < T(0));
+        // the two values the neighbour the pressure rises towards needs
+        // beyond this lane's own reach
+        const T p3 = sm.xp[own + 3 * sx], v2 = sm.xv[own + 2 * sx];
+        __syncwarp();  // every lane has read the exchange rows
+        const T chx = (T)chi_base<T>(pr1, pl1, pr2, pl2, vl1, vr1);
+        const bool upw = sx > 0;
+        const T cn = (T)chi_base<T>(upw ? pr2 : qp, upw ? qp : pl2, upw ? p3 : pr1,
+                                    upw ? pl1 : p3, upw ? qv : v2, upw ? v2 : qv);
+        const T cx = std_min(chx, sx != 0 ? cn : chx);
         const T dl = P[2] - P[0];
         const int sl = (T(0) < dl) - (dl < T(0));
         const T cl = std_min(CHA[1], sl > 0 ? CHA[2] : (sl < 0 ? CHA[0] : CHA[1]));
-        chi_v = std_min(std_min(chi_init, CX[0]), cl);
+        ch = std_min(std_min(chi_init, cx), cl) * T(0.5);
       }
-      const T ch = chi_v * T(0.5);
       Cons<T, D> a, b;
 #pragma unroll
       for (int c = 0; c < NC; ++c) {

@@ -103,9 +103,13 @@ __device__ __forceinline__ void walk_strip_2d(const SweepParams& p, T dtdh, int6
     const int64_t y_end = (y0 + ry < n1) ? y0 + ry : n1;
     // windows, index 4 = newest row k; row k - i at index 4 - i
     Cons<T, D> U[5];
-    T P[5], VX[5], VY[5];
-    T CHY[3];  // chi_y of rows k-4, k-3, k-2
+    T P[5];
+    T CHY[3] = {T(1), T(1), T(1)};  // chi_y of rows k-4, k-3, k-2
     Cons<T, D> er_prev, f_prev;
+    // the flattening's screen: keys of rows k-1 and k-2, and per row (bit i:
+    // row k-i) whether some lane may be flattened along y in the row before
+    // it or along x in it
+    uint32_t key1 = 0u, key2 = 0u, hist = 0u;
     const int64_t k_first = y0 - 3 - (S == 1 ? 1 : 0);
     const int64_t k_last = y_end + (S == 1 ? 3 : 2);
     // row k + 1 is loaded while row k is processed (global-load latency
@@ -133,8 +137,6 @@ __device__ __forceinline__ void walk_strip_2d(const SweepParams& p, T dtdh, int6
       for (int i = 0; i < 4; ++i) {
         U[i] = U[i + 1];
         P[i] = P[i + 1];
-        VX[i] = VX[i + 1];
-        VY[i] = VY[i + 1];
       }
       {
         Cons<T, D> u = pre;
@@ -149,24 +151,25 @@ __device__ __forceinline__ void walk_strip_2d(const SweepParams& p, T dtdh, int6
         const Derived<T, D> q = derive(u, gm1);
         U[4] = u;
         P[4] = q.p;
-        VX[4] = q.v[0];
-        VY[4] = q.v[1];
       }
-      // ---- y flattening base of row k - 2 (needs rows k-4..k) -----------
-      CHY[0] = CHY[1];
-      CHY[1] = CHY[2];
-      if (flat) CHY[2] = (T)chi_base<T>(P[3], P[1], P[4], P[0], VY[1], VY[3]);
+      if (flat) {
+        const uint32_t key = press_key(P[4]);
+        const bool steep = may_flatten<T>(key, key2) | may_flatten<T>(key, shfl_up(key, 2));
+        hist = 2u * hist + (__any_sync(0xffffffffu, steep) ? 1u : 0u);
+        key2 = key1;
+        key1 = key;
+        // ---- y flattening base of row k - 2 (needs rows k-4..k; bit 4: the
+        // base that leaves the window) ------------------------------------
+        if (hist & 0x1eu) {
+          CHY[0] = CHY[1];
+          CHY[1] = CHY[2];
+          CHY[2] = (T)chi_base<T>(P[3], P[1], P[4], P[0], U[1].v[3] * fl_rcp<T>(U[1].v[0]),
+                                  U[3].v[3] * fl_rcp<T>(U[3].v[0]));
+        }
+      }
       const int64_t j = k - 3;  // evolve row
       const bool evolve_row = (S == 0) ? (j >= y0) : (j >= y0 - 1);
       if (!evolve_row) continue;
-
-      // ---- x flattening base of row j on this lane ----------------------
-      const T pj = P[1], vxj = VX[1];
-      const T p_r1 = shfl_dn(pj, 1), p_l1 = shfl_up(pj, 1);
-      const T p_r2 = shfl_dn(pj, 2), p_l2 = shfl_up(pj, 2);
-      T chx = T(1);
-      if (flat) chx = (T)chi_base<T>(p_r1, p_l1, p_r2, p_l2, shfl_up(vxj, 1), shfl_dn(vxj, 1));
-      const T chx_r = shfl_dn(chx, 1), chx_l = shfl_up(chx, 1);
 
       // ---- evolved face states of (lane, j) -------------------------------
       const Cons<T, D>& u = U[1];
@@ -175,17 +178,23 @@ __device__ __forceinline__ void walk_strip_2d(const SweepParams& p, T dtdh, int6
         er = u;
         el = u;
       } else {
-        T chi_v = T(1);
-        if (flat) {
+        T ch = T(0.5);
+        if (flat && (hist & 0xeu) != 0u) {
+          // ---- x flattening base of row j on this lane --------------------
+          const T pj = P[1], vxj = u.v[2] * fl_rcp<T>(u.v[0]);
+          const T p_r1 = shfl_dn(pj, 1), p_l1 = shfl_up(pj, 1);
+          const T p_r2 = shfl_dn(pj, 2), p_l2 = shfl_up(pj, 2);
+          const T chx =
+              (T)chi_base<T>(p_r1, p_l1, p_r2, p_l2, shfl_up(vxj, 1), shfl_dn(vxj, 1));
+          const T chx_r = shfl_dn(chx, 1), chx_l = shfl_up(chx, 1);
           const T dx = p_r1 - p_l1;
           const int sx = (T(0) < dx) - (dx < T(0));
           const T cx = std_min(chx, sx > 0 ? chx_r : (sx < 0 ? chx_l : chx));
           const T dy = P[2] - P[0];
           const int sy = (T(0) < dy) - (dy < T(0));
           const T cy = std_min(CHY[1], sy > 0 ? CHY[2] : (sy < 0 ? CHY[0] : CHY[1]));
-          chi_v = std_min(std_min(chi_init, cx), cy);
+          ch = std_min(std_min(chi_init, cx), cy) * T(0.5);
         }
-        const T ch = chi_v * T(0.5);
         Cons<T, D> a, b;
         // the limiter kind tested once per position, not per component
         auto slopes = [&](auto lim) {

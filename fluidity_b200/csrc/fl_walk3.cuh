@@ -92,12 +92,12 @@ __device__ __forceinline__ void walk_strip_3d(const SweepParams& p, const T* __r
   const int64_t y_end = (y0 + ry < nr) ? y0 + ry : nr;
   // windows, index 4 = newest row k; row k - i at index 4 - i
   Cons<T, D> U[5];
-  // FP64 re-derives the velocities the flattening needs from U (two more
-  // reciprocals per row, 16 fewer live registers, fewer spills: +7%); FP32
-  // keeps them in windows (re-deriving measured 1.5% slower there)
-  constexpr bool kRederive = sizeof(T) == 8;
-  T P[5], VX[5], VY[5];
-  T CHY[3];  // row-direction chi bases of rows k-4, k-3, k-2
+  T P[5];
+  T CHY[3] = {T(1), T(1), T(1)};  // row-direction chi bases of rows k-4, k-3, k-2
+  // the flattening's screen: keys of rows k-1 and k-2, and per row (bit i: row
+  // k-i) whether some lane may be flattened along the rows in the row before
+  // it or along x in it
+  uint32_t key1 = 0u, key2 = 0u, hist = 0u;
   Cons<T, D> er_prev, f_prev;
   const int64_t k_first = y0 - 3 - SW;
   const int64_t k_last = y_end + 2 + SW;
@@ -134,10 +134,6 @@ __device__ __forceinline__ void walk_strip_3d(const SweepParams& p, const T* __r
     for (int i = 0; i < 4; ++i) {
       U[i] = U[i + 1];
       P[i] = P[i + 1];
-      if constexpr (!kRederive) {
-        VX[i] = VX[i + 1];
-        VY[i] = VY[i + 1];
-      }
     }
     {
       Cons<T, D> u = pre;
@@ -152,33 +148,24 @@ __device__ __forceinline__ void walk_strip_3d(const SweepParams& p, const T* __r
       const Derived<T, D> q = derive(u, gm1);
       U[4] = u;
       P[4] = q.p;
-      if constexpr (!kRederive) {
-        VX[4] = q.v[0];
-        VY[4] = q.v[DR];
-      }
     }
-    CHY[0] = CHY[1];
-    CHY[1] = CHY[2];
-    // re-derived: the same products derive() formed when the rows were loaded
-    const T rinv1 = kRederive ? fl_rcp<T>(U[1].v[0]) : T(0);
     if (flat) {
-      if constexpr (kRederive)
-        CHY[2] = (T)chi_base<T>(P[3], P[1], P[4], P[0], U[1].v[2 + DR] * rinv1,
+      const uint32_t key = press_key(P[4]);
+      const bool steep = may_flatten<T>(key, key2) | may_flatten<T>(key, shfl_up(key, 2));
+      hist = 2u * hist + (__any_sync(0xffffffffu, steep) ? 1u : 0u);
+      key2 = key1;
+      key1 = key;
+      // the base of row k - 2 (bit 4: the base that leaves the window)
+      if (hist & 0x1eu) {
+        CHY[0] = CHY[1];
+        CHY[1] = CHY[2];
+        CHY[2] = (T)chi_base<T>(P[3], P[1], P[4], P[0], U[1].v[2 + DR] * fl_rcp<T>(U[1].v[0]),
                                 U[3].v[2 + DR] * fl_rcp<T>(U[3].v[0]));
-      else
-        CHY[2] = (T)chi_base<T>(P[3], P[1], P[4], P[0], VY[1], VY[3]);
+      }
     }
     const int64_t j = k - 3;  // evolve row
     const bool evolve_row = (SW == 0) ? (j >= y0) : (j >= y0 - 1);
     if (!evolve_row) continue;
-
-    // ---- x flattening base of row j on this lane --------------------------
-    const T pj = P[1], vxj = kRederive ? U[1].v[2] * rinv1 : VX[1];
-    const T p_r1 = shfl_dn(pj, 1), p_l1 = shfl_up(pj, 1);
-    const T p_r2 = shfl_dn(pj, 2), p_l2 = shfl_up(pj, 2);
-    T chx = T(1);
-    if (flat) chx = (T)chi_base<T>(p_r1, p_l1, p_r2, p_l2, shfl_up(vxj, 1), shfl_dn(vxj, 1));
-    const T chx_r = shfl_dn(chx, 1), chx_l = shfl_up(chx, 1);
 
     const Cons<T, D>& u = U[1];
     Cons<T, D> er, el;
@@ -186,19 +173,27 @@ __device__ __forceinline__ void walk_strip_3d(const SweepParams& p, const T* __r
       er = u;
       el = u;
     } else {
-      T chi_v = T(1);
+      T ch = T(0.5);
       if (flat) {
-        const T dx = p_r1 - p_l1;
-        const int sx = (T(0) < dx) - (dx < T(0));
-        const T cx = std_min(chx, sx > 0 ? chx_r : (sx < 0 ? chx_l : chx));
-        const T dy = P[2] - P[0];
-        const int sy = (T(0) < dy) - (dy < T(0));
-        const T cr = std_min(CHY[1], sy > 0 ? CHY[2] : (sy < 0 ? CHY[0] : CHY[1]));
+        T cx = T(1), cr = T(1);
+        if ((hist & 0xeu) != 0u) {
+          // ---- x flattening base of row j on this lane --------------------
+          const T pj = P[1], vxj = u.v[2] * fl_rcp<T>(u.v[0]);
+          const T p_r1 = shfl_dn(pj, 1), p_l1 = shfl_up(pj, 1);
+          const T p_r2 = shfl_dn(pj, 2), p_l2 = shfl_up(pj, 2);
+          const T chx =
+              (T)chi_base<T>(p_r1, p_l1, p_r2, p_l2, shfl_up(vxj, 1), shfl_dn(vxj, 1));
+          const T chx_r = shfl_dn(chx, 1), chx_l = shfl_up(chx, 1);
+          const T dx = p_r1 - p_l1;
+          const int sx = (T(0) < dx) - (dx < T(0));
+          cx = std_min(chi_init, std_min(chx, sx > 0 ? chx_r : (sx < 0 ? chx_l : chx)));
+          const T dy = P[2] - P[0];
+          const int sy = (T(0) < dy) - (dy < T(0));
+          cr = std_min(CHY[1], sy > 0 ? CHY[2] : (sy < 0 ? CHY[0] : CHY[1]));
+        }
         // minimum over dimensions 0, 1, 2 in order
-        chi_v = (DR == 1) ? std_min(std_min(std_min(chi_init, cx), cr), ct)
-                          : std_min(std_min(std_min(chi_init, cx), ct), cr);
+        ch = T(0.5) * ((DR == 1) ? std_min(std_min(cx, cr), ct) : std_min(std_min(cx, ct), cr));
       }
-      const T ch = chi_v * T(0.5);
       Cons<T, D> a, b;
       // the limiter kind tested once per position, not per component
       auto slopes = [&](auto lim) {
@@ -362,6 +357,7 @@ chi_dim_kernel(SweepParams p, T* __restrict__ xc, int ry) {
   for (int64_t pl = blockIdx.z; pl < p.n[DR]; pl += gridDim.z) {
     const int64_t base = pl * ps;
     T P[5], V[5], CH[3];
+    uint32_t key1 = 0u, key2 = 0u, hist = 0u;  // bit i: row k-1-i may be flattened
     for (int64_t k = j0 - 3; k <= j_end + 2; ++k) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -379,7 +375,12 @@ chi_dim_kernel(SweepParams p, T* __restrict__ xc, int ry) {
       V[4] = q.v[DT];
       CH[0] = CH[1];
       CH[1] = CH[2];
-      CH[2] = (T)chi_base<T>(P[3], P[1], P[4], P[0], V[1], V[3]);  // base of row k - 2
+      const uint32_t key = press_key(q.p);
+      hist = 2u * hist + (may_flatten<T>(key, key2) ? 1u : 0u);
+      key2 = key1;
+      key1 = key;
+      CH[2] = T(1);
+      if (hist & 2u) CH[2] = (T)chi_base<T>(P[3], P[1], P[4], P[0], V[1], V[3]);  // of row k - 2
       const int64_t j = k - 3;
       if (j < j0 || x >= n0) continue;
       const T dt = P[2] - P[0];

@@ -254,6 +254,41 @@ def test_strip_lengths_match_oracle(cuda, oracle, shape, dtype):
         assert abs(ws - top) < 10 * TOL[dtype] * top, dim
 
 
+def oblique_shock(shape, width):
+    """Compression fronts `width` cells wide at two angles, so that every
+    column, row and plane of the grid has a cell on the flattening's ramp,
+    among flow far from it."""
+    x = np.meshgrid(*[np.arange(n) + 0.5 for n in shape[::-1]], indexing="ij")[::-1]
+    s = x[0] + 0.61 * x[1] + (0.37 * x[2] if len(shape) > 2 else 0.0)
+    t = x[0] - 0.83 * x[1]
+    front = np.tanh((s - 0.6 * shape[0]) / width) + 0.6 * np.tanh((t - 0.2 * shape[0]) / width)
+    prim = np.zeros((len(shape) + 2, int(np.prod(shape))))
+    prim[0] = (1.5 - 0.4 * front).reshape(-1)
+    prim[1] = (2.2 - 1.2 * front).reshape(-1)
+    for d in range(len(shape)):
+        prim[2 + d] = (-0.5 * front / (d + 1)).reshape(-1)
+    return prim
+
+
+@pytest.mark.parametrize("shape", [(88, 61), (31, 90), (45, 38, 20)],
+                         ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("reflect", [False, True])
+def test_flattening_screen_at_every_lane(cuda, oracle, shape, dtype, reflect):
+    """The walks skip the flattening where their screen rules it out for the
+    whole warp; a front that crosses every lane, strip and plane must be
+    flattened exactly as the oracle flattens it."""
+    u = oracle.prim_to_cons(oblique_shock(shape, 1.3), GAMMA, dtype=NPDT[dtype])
+    mask = 2 ** len(shape) - 1 if reflect else 0
+    for dim in range(len(shape)):
+        args = (shape, dim, u, NPDT[dtype](GAMMA), NPDT[dtype](0.05))
+        want = oracle.sweep(*args, reflect=mask)
+        plain = oracle.sweep(*args, reflect=mask, flatten=False)
+        assert err(plain, want, dtype) > 1e-3     # the front is flattened
+        got = gpu_sweep(shape, dim, u, 0.05, dtype=dtype, reflect=mask)
+        assert err(got, want, dtype) < TOL[dtype], dim
+
+
 @pytest.mark.parametrize("shape", [(100001,), (317, 211), (37, 29, 23)],
                          ids=lambda s: "x".join(map(str, s)))
 @pytest.mark.parametrize("where", ["first", "middle", "last"])
