@@ -213,21 +213,6 @@ FL_HD void riemann(const Cons<T, D>& ul, const Cons<T, D>& ur, int d,
   }
 }
 
-// ---- limiters (limiting/van_leer_limiter.hpp:65-74, superbee 72-89) -----
-
-template <typename T>
-FL_HD T limit_single(int limiter, T left, T right) {
-  const T r = left / right;
-  if (limiter == kSuperbee) {
-    if (r <= T(0) || right == T(0)) return T(0);
-    if (r <= T(0.5)) return T(2) * r;
-    if (r <= T(1)) return T(1);
-    const T er = T(2) / (T(1) + r);
-    return std_min(er, std_min(r, T(2)));
-  }
-  return (r <= T(0) || right == T(0)) ? T(0) : T(2) * std_min(r, T(1)) / (T(1) + r);
-}
-
 // FL_FAST_DIV 1 (the default): the HLLC star speed, star scale, energy
 // term and shock pressure ratios multiply by one reciprocal instead of
 // dividing, and the flattening threshold test compares a product; results
@@ -560,15 +545,21 @@ FL_HD void riemann_q(const Cons<T, D>& ul, const Derived<T, D>& ql,
   riemann_qh<FLUX>(ul, ql, ur, qr, d, gamma, gm1, adi, dtdh, T(1.0) / dtdh, f, pinf);
 }
 
-// The reference's van Leer slope 0.5 (bd + fd) * 2 min(r, 1) / (1 + r) with
-// r = bd / fd equals, in exact arithmetic, minmod(bd, fd): bd when
-// 0 < r <= 1, fd when r > 1, 0 when r <= 0 or fd == 0.  Superbee keeps the
-// reference's formula.
+// The limited slopes 0.5 (bd + fd) phi(r), r = bd / fd, without the
+// limiters' divisions (exact arithmetic; the results differ by rounding).
+// van Leer, phi = 2 min(r, 1) / (1 + r): minmod(bd, fd), that is bd when
+// 0 < r <= 1, fd when r > 1, 0 when r <= 0 or fd == 0.  Superbee: r (bd + fd)
+// when 0 < r <= 1/2, the mean when r <= 1, and above 1, where phi = 2 / (1 + r)
+// is the least of its three terms, fd; only the first range needs r, by a
+// reciprocal.  With this form and the walks' common loop compiled for superbee
+// too, the 257 x 191 FP64 FORCE step between walls took 30 instead of 41 us
+// and the 600^2 FP64 HLLC step 72 instead of 90 us.
 template <typename T>
 FL_HD T limited_slope(int limiter, T bd, T fd) {
   if (limiter == kSuperbee) {
-    T lim = T(0.5) * (bd + fd);
-    return lim * limit_single<T>(kSuperbee, bd, fd);
+    const T ab = fl_abs<T>(bd), af = fl_abs<T>(fd), sum = bd + fd;
+    const T below = ab <= T(0.5) * af ? bd * fl_rcp<T>(fd) * sum : T(0.5) * sum;
+    return (bd * fd > T(0)) ? (ab <= af ? below : fd) : T(0) * sum;  // NaN stays
   }
   // one product and test for "the same sign, neither zero" (false for NaN);
   // slopes whose product underflows (below 4e-23 in FP32, 2e-162 in FP64)

@@ -121,13 +121,14 @@ __device__ __forceinline__ void walk_strip_2d(const SweepParams& p, T dtdh, int6
 #pragma unroll
       for (int c = 0; c < NC; ++c) pre.v[c] = __ldg(in + c * pitch + gy * n0 + gx);
     }
-    // the walk; its common form (FAST: no reflective end in x or y, MUSCL
-    // with flattening and the van Leer limiter, the wavespeed in the y sweep
-    // only) has the reflective flips and the reconstruction, limiter and
-    // wavespeed tests compiled out.  A slab's row window for the wavespeed
+    // the walk, with the limiter kind fixed for the whole strip; its common
+    // form (FAST: no reflective end in x or y, MUSCL with flattening, the
+    // wavespeed in the y sweep only) has the reflective flips and the
+    // reconstruction and wavespeed tests compiled out.  A slab's row window for the wavespeed
     // stays a runtime test, so that slabs take the same code as the
     // undivided grid and match it bit for bit.
-    auto walk = [&](auto fast) {
+    auto walk = [&](auto lim, auto fast) {
+    constexpr int LIM = decltype(lim)::value;
     constexpr bool FAST = decltype(fast)::value;
     const bool flat = FAST || flatten;
     const bool mus = FAST || muscl;
@@ -196,28 +197,20 @@ __device__ __forceinline__ void walk_strip_2d(const SweepParams& p, T dtdh, int6
           ch = std_min(std_min(chi_init, cx), cy) * T(0.5);
         }
         Cons<T, D> a, b;
-        // the limiter kind tested once per position, not per component
-        auto slopes = [&](auto lim) {
 #pragma unroll
-          for (int c = 0; c < NC; ++c) {
-            T um, up;
-            if (S == 0) {
-              um = shfl_up(u.v[c], 1);
-              up = shfl_dn(u.v[c], 1);
-            } else {
-              um = U[0].v[c];
-              up = U[2].v[c];
-            }
-            const T delta =
-                ch * limited_slope<T>(decltype(lim)::value, u.v[c] - um, up - u.v[c]);
-            a.v[c] = u.v[c] - delta;
-            b.v[c] = u.v[c] + delta;
+        for (int c = 0; c < NC; ++c) {
+          T um, up;
+          if (S == 0) {
+            um = shfl_up(u.v[c], 1);
+            up = shfl_dn(u.v[c], 1);
+          } else {
+            um = U[0].v[c];
+            up = U[2].v[c];
           }
-        };
-        if (!FAST && p.limiter == kSuperbee)
-          slopes(std::integral_constant<int, kSuperbee>{});
-        else
-          slopes(std::integral_constant<int, kVanLeer>{});
+          const T delta = ch * limited_slope<T>(LIM, u.v[c] - um, up - u.v[c]);
+          a.v[c] = u.v[c] - delta;
+          b.v[c] = u.v[c] + delta;
+        }
         Cons<T, D> fa, fb;
         flux_q(a, derive(a, gm1), S, fa);
         flux_q(b, derive(b, gm1), S, fb);
@@ -272,10 +265,16 @@ __device__ __forceinline__ void walk_strip_2d(const SweepParams& p, T dtdh, int6
       }
     }
     };
-    if ((p.reflect & 3u) == 0 && flatten && p.limiter == kVanLeer && want_ws == (S == 1))
-      walk(std::true_type{});
-    else
-      walk(std::false_type{});
+    using SB = std::integral_constant<int, kSuperbee>;
+    using VL = std::integral_constant<int, kVanLeer>;
+    const bool fast = (p.reflect & 3u) == 0 && flatten && want_ws == (S == 1);
+    if (p.limiter == kSuperbee) {
+      if (fast) walk(SB{}, std::true_type{});
+      else walk(SB{}, std::false_type{});
+    } else {
+      if (fast) walk(VL{}, std::true_type{});
+      else walk(VL{}, std::false_type{});
+    }
   }
 }
 

@@ -254,6 +254,31 @@ def test_strip_lengths_match_oracle(cuda, oracle, shape, dtype):
         assert abs(ws - top) < 10 * TOL[dtype] * top, dim
 
 
+@pytest.mark.parametrize("shape", [(97,), (70, 33), (30, 21, 9)],
+                         ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("reflect", [False, True])
+def test_superbee_slope_ranges(cuda, oracle, shape, dtype, reflect):
+    """Superbee's slope takes one of four forms by the ratio r of the one-sided
+    differences (r <= 0, to 1/2, to 1, above): fields with differences of both
+    signs, zero and of the ratios 1/2, 1 and 2 exactly, with the common and the
+    walled form of the walks, against the oracle's division form."""
+    rng = np.random.default_rng(3)
+    n = int(np.prod(shape))
+    prim = np.zeros((len(shape) + 2, n))
+    prim[0] = 2.0 + rng.integers(0, 5, n) / 8.0          # exact differences k / 8
+    prim[1] = 1.5 + rng.integers(0, 5, n) / 16.0
+    for d in range(len(shape)):
+        prim[2 + d] = rng.integers(-2, 3, n) / 16.0
+    u = oracle.prim_to_cons(prim, GAMMA, dtype=NPDT[dtype])
+    mask = 2 ** len(shape) - 1 if reflect else 0
+    for dim in range(len(shape)):
+        want = oracle.sweep(shape, dim, u, NPDT[dtype](GAMMA), NPDT[dtype](0.05),
+                            limiter="superbee", reflect=mask)
+        got = gpu_sweep(shape, dim, u, 0.05, dtype=dtype, limiter="superbee", reflect=mask)
+        assert err(got, want, dtype) < TOL[dtype], dim
+
+
 def oblique_shock(shape, width):
     """Compression fronts `width` cells wide at two angles, so that every
     column, row and plane of the grid has a cell on the flattening's ramp,
