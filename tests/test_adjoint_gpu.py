@@ -91,6 +91,40 @@ def test_adjoint_sweep_reflective_walls(cuda, seed, dim, flux):
     assert abs(fd - ad) <= 1e-6 * max(abs(ad), 1e-12), (fd, ad)
 
 
+@pytest.mark.parametrize("shape", [(27, 9), (28, 8), (29, 17), (57, 30), (8, 28), (9, 29), (4, 57)],
+                         ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("dim", [0, 1])
+@pytest.mark.parametrize("flux", ["hllc", "force"])
+@pytest.mark.parametrize("reflect", [0, 3])
+def test_adjoint_sweep_tile_edges(cuda, oracle, shape, dim, flux, reflect):
+    """Grids of one 28 x 8 tile, just below and above it and with remainders in
+    both directions: <J^T lam, du> = <lam, J du>, J du from the oracle's dual
+    numbers (the same frozen branches, so equal to rounding: the bound is
+    1e-11 of the sum of the terms' magnitudes)."""
+    import torch
+    from fluidity_b200 import capi
+    from fluidity_b200.solver import SplitSolver
+    lib = capi.load()
+    u = _smooth_state(shape, 7)
+    s = SplitSolver(shape, flux=flux, gamma=GAMMA, boundary_mask=reflect, flatten=False)
+    d = torch.from_numpy(u).cuda()
+    dtdh = 0.6 / s.max_wavespeed(d).item()
+    rng = np.random.default_rng(17)
+    lam = rng.standard_normal(u.shape)
+    du = 1e-2 * rng.standard_normal(u.shape) * np.abs(u)
+    _, dout = oracle.sweep_dual(shape, dim, u, du, GAMMA, dtdh, flux=flux, reflect=reflect,
+                                flatten=False)
+    dl = torch.from_numpy(lam).cuda()
+    lam_in = torch.empty_like(d)
+    capi.check(lib.fl_adjoint_sweep(C.byref(s.grid), dim, C.c_void_p(d.data_ptr()),
+                                    C.c_void_p(dl.data_ptr()), C.c_void_p(lam_in.data_ptr()),
+                                    GAMMA, dtdh, s.policy, reflect, None))
+    torch.cuda.synchronize()
+    got = float(np.sum(lam_in.cpu().numpy() * du))
+    want = float(np.sum(lam * dout))
+    assert abs(got - want) <= 1e-11 * float(np.sum(np.abs(lam * dout))), (got, want)
+
+
 def _smooth_density(n, seed):
     """1 + a few low Fourier modes: smooth everywhere, no flat regions."""
     import torch
