@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -23,7 +24,7 @@ int bfail(int code, const char* fmt, A... args) {
 
 // 1-D size classes: CTA width per class (autotuned), upper n per class.
 constexpr int kClasses = 3;
-constexpr int kClassThreads[3] = {128, 256, 512};
+
 
 }  // namespace
 }  // namespace fl
@@ -57,11 +58,12 @@ struct fl_batch {
   // autotuned: 1-D class boundaries (n <= bound -> class) and 2-D strip rows
   int bound1d[2] = {512, 2048};
   int ry_small = 32, ry_mid = 64, ry_large = 64;   // side <= 128, <= 256, larger
+  bool tuned = false;           // the rows above are the autotuner's
   void* arena_a = nullptr;
   void* arena_b = nullptr;
-  cudaStream_t side = nullptr;
+  cudaStream_t side[kClasses] = {nullptr, nullptr, nullptr};  // one per 1-D class
   cudaStream_t cap = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join[kClasses] = {nullptr, nullptr, nullptr};
   cudaGraphExec_t graph = nullptr;
   int64_t graph_steps = 0;
 };
@@ -76,6 +78,48 @@ int pick_ry(const fl_batch* b, int64_t side) {
   return side <= 128 ? b->ry_small : (side <= 256 ? b->ry_mid : b->ry_large);
 }
 
+// Strips of a 2-D problem of n1 rows, at most ry rows each.
+int64_t strip_count(int64_t n1, int ry) { return (n1 + ry - 1) / ry; }
+
+// Upper bound on the strip rows of an untuned plan, by the estimated time of
+// a sweep over all the batch's 2-D problems (the estimate of strip_rows in
+// fl_sweep_dispatch.inc): batches that cannot fill the resident warps run at
+// the latency of one strip, so they take short ones; batches of several
+// rounds keep 64 rows, which waste least on the halo.  The batches
+// and figures at batch1d_kernel include it.
+int strip_cap(const fl_batch* b) {
+  constexpr double kAlone = 5.0, kShared = 1.5;
+  constexpr int kHalo = 7;
+  using W = WalkCfg<float, 0>;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const double slots = (double)sms * W::WARPS * (b->f32 ? 5 : 3);
+  int best = 64;
+  double best_t = 0.0;
+  for (int cap = 64; cap >= 8; cap /= 2) {
+    double items = 0.0, positions = 0.0;
+    int64_t longest = 0;
+    for (const fl_batch_desc& d : b->desc) {
+      if (d.dims != 2) continue;
+      const int ry = std::min(pick_ry(b, std::max(d.n[0], d.n[1])), cap);
+      const int64_t cols = (d.n[0] + W::OWN - 1) / W::OWN, ns = strip_count(d.n[1], ry);
+      items += (double)(cols * ns);
+      positions += (double)(cols * (d.n[1] + ns * kHalo));
+      longest = std::max(longest, (d.n[1] + ns - 1) / ns + kHalo);
+    }
+    const double per = std::ceil(items / (4.0 * sms));
+    const double t = items <= slots
+                         ? (double)longest * std::max(kAlone, per * kShared)
+                         : positions * kShared / (4.0 * sms) + 0.5 * kAlone * (double)longest;
+    if (cap == 64 || t < best_t) {
+      best = cap;
+      best_t = t;
+    }
+  }
+  return best;
+}
+
 int pick_class(const fl_batch* b, int64_t n) {
   return n <= b->bound1d[0] ? 0 : (n <= b->bound1d[1] ? 1 : 2);
 }
@@ -87,6 +131,7 @@ int upload_plan(fl_batch* b) {
   std::vector<BatchProblem> pr(n);
   std::vector<BatchItem> items;
   std::vector<int> cls_lists[kClasses];
+  const int cap = b->tuned ? 1 << 30 : strip_cap(b);
   for (int i = 0; i < n; ++i) {
     const fl_batch_desc& d = b->desc[i];
     BatchProblem& p = pr[i];
@@ -99,7 +144,10 @@ int upload_plan(fl_batch* b) {
     if (d.dims == 1) {
       cls_lists[pick_class(b, d.n[0])].push_back(i);
     } else {
-      const int ry = pick_ry(b, std::max(d.n[0], d.n[1]));
+      // the rows evenly over the strips: the stacked warps of a CTA, and the
+      // CTAs of a problem, end together
+      const int64_t ns = strip_count(d.n[1], std::min(pick_ry(b, std::max(d.n[0], d.n[1])), cap));
+      const int ry = (int)((d.n[1] + ns - 1) / ns);
       p.ry = ry;
       using W = WalkCfg<float, 0>;   // the x sweep owns fewer columns: size by it
       const int64_t bx = (d.n[0] + W::OWN - 1) / W::OWN;
@@ -167,11 +215,11 @@ BatchArgs base_args(const fl_batch* b) {
   return a;
 }
 
-template <typename T, int FLUX, int THREADS>
+template <typename T, int FLUX>
 cudaError_t set_attr_1d() {
   // the largest 1-D problem that fits
   const size_t smem = 2 * 3 * (size_t)(batch1d_max<T>() + 8) * sizeof(T);
-  return cudaFuncSetAttribute(batch1d_kernel<T, FLUX, THREADS>,
+  return cudaFuncSetAttribute(batch1d_kernel<T, FLUX>,
                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
@@ -183,13 +231,8 @@ cudaError_t prepare(const fl_batch* b) {
   if (e != cudaSuccess) return e;
   if (dev < 64 && done[dev]) return cudaSuccess;
   constexpr int kSH = kHllc | kStiffEos, kSF = kForce | kStiffEos;
-  const cudaError_t r[] = {
-      set_attr_1d<T, kHllc, 64>(), set_attr_1d<T, kHllc, 128>(), set_attr_1d<T, kHllc, 256>(),
-      set_attr_1d<T, kHllc, 512>(), set_attr_1d<T, kForce, 64>(), set_attr_1d<T, kForce, 128>(),
-      set_attr_1d<T, kForce, 256>(), set_attr_1d<T, kForce, 512>(),
-      set_attr_1d<T, kSH, 64>(), set_attr_1d<T, kSH, 128>(), set_attr_1d<T, kSH, 256>(),
-      set_attr_1d<T, kSH, 512>(), set_attr_1d<T, kSF, 64>(), set_attr_1d<T, kSF, 128>(),
-      set_attr_1d<T, kSF, 256>(), set_attr_1d<T, kSF, 512>()};
+  const cudaError_t r[] = {set_attr_1d<T, kHllc>(), set_attr_1d<T, kForce>(),
+                           set_attr_1d<T, kSH>(), set_attr_1d<T, kSF>()};
   for (cudaError_t x : r)
     if (x != cudaSuccess) return x;
   if (dev < 64) done[dev] = true;
@@ -197,36 +240,27 @@ cudaError_t prepare(const fl_batch* b) {
   return cudaSuccess;
 }
 
-template <typename T, int FLUX, int THREADS>
+template <typename T, int FLUX>
 cudaError_t launch_1d(const fl_batch* b, int c, int64_t nsteps, cudaStream_t st) {
+  const int threads = b->cls_threads[c];
   BatchArgs a = base_args(b);
   a.order = b->d_order + b->cls_first[c];
   a.count = b->cls_count[c];
   a.queue = b->d_queue + c;
   const int ld = b->cls_nmax[c] + 8;
   const size_t smem = 2 * 3 * (size_t)ld * sizeof(T);
-  auto k = batch1d_kernel<T, FLUX, THREADS>;
+  auto k = batch1d_kernel<T, FLUX>;
   cudaError_t e = prepare<T>(b);
   if (e != cudaSuccess) return e;
   batch_reset_queue_kernel<<<1, 1, 0, st>>>(a.queue);
   int dev = 0, sms = 148, per_sm = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, THREADS, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem);
   int grid = sms * std::max(per_sm, 1);
   grid = std::min(grid, a.count);
-  k<<<grid, THREADS, smem, st>>>(a, (long long)nsteps, ld);
+  k<<<grid, threads, smem, st>>>(a, (long long)nsteps, ld);
   return cudaGetLastError();
-}
-
-template <typename T, int FLUX>
-cudaError_t launch_1d_class(const fl_batch* b, int c, int64_t nsteps, cudaStream_t st) {
-  switch (b->cls_threads[c]) {
-    case 64: return launch_1d<T, FLUX, 64>(b, c, nsteps, st);
-    case 128: return launch_1d<T, FLUX, 128>(b, c, nsteps, st);
-    case 256: return launch_1d<T, FLUX, 256>(b, c, nsteps, st);
-    default: return launch_1d<T, FLUX, 512>(b, c, nsteps, st);
-  }
 }
 
 template <typename T, int FLUX>
@@ -243,25 +277,27 @@ cudaError_t launch_2d_step(const fl_batch* b, cudaStream_t st) {
 template <typename T, int FLUX>
 cudaError_t enqueue_steps(fl_batch* b, int64_t nsteps, cudaStream_t st, bool do1d, bool do2d) {
   cudaError_t e = cudaSuccess;
-  const bool has1d = do1d && (b->cls_count[0] + b->cls_count[1] + b->cls_count[2]) > 0;
   const bool has2d = do2d && b->n_items > 0;
-  if (has1d && has2d) {
-    // fork the resident 1-D launches onto the side stream
-    if ((e = cudaEventRecord(b->ev_fork, st)) != cudaSuccess) return e;
-    if ((e = cudaStreamWaitEvent(b->side, b->ev_fork, 0)) != cudaSuccess) return e;
+  int parts = has2d ? 1 : 0;
+  for (int c = 0; c < kClasses; ++c) parts += (do1d && b->cls_count[c] > 0) ? 1 : 0;
+  // the 1-D classes' resident launches run beside each other and beside the
+  // 2-D sweeps, each on a stream of its own
+  const bool fork = parts > 1;
+  if (fork && (e = cudaEventRecord(b->ev_fork, st)) != cudaSuccess) return e;
+  for (int c = 0; do1d && c < kClasses; ++c) {
+    if (b->cls_count[c] == 0) continue;
+    cudaStream_t s1 = fork ? b->side[c] : st;
+    if (fork && (e = cudaStreamWaitEvent(s1, b->ev_fork, 0)) != cudaSuccess) return e;
+    e = launch_1d<T, FLUX>(b, c, nsteps, s1);
+    if (e == cudaSuccess && fork) e = cudaEventRecord(b->ev_join[c], s1);
+    if (e != cudaSuccess) return e;
   }
-  cudaStream_t s1 = (has1d && has2d) ? b->side : st;
-  if (has1d)
-    for (int c = 0; c < kClasses; ++c)
-      if (b->cls_count[c] > 0 && (e = launch_1d_class<T, FLUX>(b, c, nsteps, s1)) != cudaSuccess)
-        return e;
   if (has2d)
     for (int64_t s = 0; s < nsteps; ++s)
       if ((e = launch_2d_step<T, FLUX>(b, st)) != cudaSuccess) return e;
-  if (has1d && has2d) {
-    if ((e = cudaEventRecord(b->ev_join, b->side)) != cudaSuccess) return e;
-    if ((e = cudaStreamWaitEvent(st, b->ev_join, 0)) != cudaSuccess) return e;
-  }
+  for (int c = 0; fork && do1d && c < kClasses; ++c)
+    if (b->cls_count[c] > 0 && (e = cudaStreamWaitEvent(st, b->ev_join[c], 0)) != cudaSuccess)
+      return e;
   return cudaSuccess;
 }
 
@@ -333,10 +369,12 @@ int fl_batch_create(fl_batch** out, const fl_batch_desc* problems, int32_t count
   if (e == cudaSuccess) e = cudaMalloc(&b->d_res, count * sizeof(double));
   if (e == cudaSuccess) e = cudaMemcpy(b->d_res, res.data(), count * sizeof(double), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemset(b->d_ctrl, 0, count * sizeof(StepControl));
-  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking);
+  for (int c = 0; c < kClasses; ++c) {
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->side[c], cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_join[c], cudaEventDisableTiming);
+  }
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming);
   if (e != cudaSuccess) {
     fl_batch_destroy(b);
     return bfail(kENoMem, "fl_batch_create: %s", cudaGetErrorString(e));
@@ -359,10 +397,12 @@ int fl_batch_destroy(fl_batch* b) {
   cudaFree(b->d_order);
   cudaFree(b->d_queue);
   cudaFree(b->d_res);
-  if (b->side) cudaStreamDestroy(b->side);
+  for (int c = 0; c < kClasses; ++c) {
+    if (b->side[c]) cudaStreamDestroy(b->side[c]);
+    if (b->ev_join[c]) cudaEventDestroy(b->ev_join[c]);
+  }
   if (b->cap) cudaStreamDestroy(b->cap);
   if (b->ev_fork) cudaEventDestroy(b->ev_fork);
-  if (b->ev_join) cudaEventDestroy(b->ev_join);
   delete b;
   return kOk;
 }
@@ -530,6 +570,7 @@ int fl_batch_autotune(fl_batch* b, void* arena_a, void* arena_b, int64_t trial_s
   }
   // 2-D: strip rows per size class (small / mid / large sides)
   if (b->n_items > 0) {
+    b->tuned = true;
     int* slots[3] = {&b->ry_small, &b->ry_mid, &b->ry_large};
     for (int c = 0; c < 3; ++c) {
       float best = 1e30f;

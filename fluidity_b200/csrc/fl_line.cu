@@ -32,6 +32,7 @@
 
 #include "fl_internal.cuh"
 #include "fl_launch.cuh"
+#include "fl_line_cell.cuh"
 #include "fl_numerics.cuh"
 #include "fl_sweep.cuh"
 
@@ -40,7 +41,7 @@ namespace cg = cooperative_groups;
 namespace fl {
 namespace {
 
-constexpr int kOwn = 24;       // cells a warp updates
+constexpr int kOwn = kLineOwn;  // cells a warp updates
 constexpr int kMaxWarps = 20;  // 640 threads: up to 96 registers each
 constexpr int kMaxCluster = 8;
 
@@ -54,64 +55,6 @@ __device__ __forceinline__ double warp_max_bits(double v) {
   const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
   const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
   return __hiloint2double((int)mh, (int)ml);
-}
-
-template <typename T>
-__device__ __forceinline__ T up(T v, int d) { return __shfl_up_sync(0xffffffffu, v, d); }
-template <typename T>
-__device__ __forceinline__ T dn(T v, int d) { return __shfl_down_sync(0xffffffffu, v, d); }
-
-// New state of this lane's cell (valid on lanes 4..27), x its index in the
-// planes of `src` (plane stride ld).
-template <typename T, int FLUX, int LIM, bool MUSCL, bool FLAT>
-__device__ __forceinline__ Cons<T, 1> line_cell(const T* src, int ld, int x, T gamma, T gm1, T adi,
-                                                T dtdh, T dhdt, T pinf) {
-  constexpr int NC = 3;
-  Cons<T, 1> u, er, el;
-#pragma unroll
-  for (int c = 0; c < NC; ++c) u.v[c] = src[c * ld + x];
-  if constexpr (MUSCL) {
-    T ch = T(0.5);
-    if constexpr (FLAT) {
-      const Derived<T, 1> q = derive(u, gm1);
-      const T pr = dn(q.p, 1), pl = up(q.p, 1);
-      const T base = (T)chi_base<T>(pr, pl, dn(q.p, 2), up(q.p, 2), up(q.v[0], 1), dn(q.v[0], 1));
-      const T br = dn(base, 1), bl = up(base, 1);
-      const T dx = pr - pl;
-      ch *= std_min(base, dx > T(0) ? br : (dx < T(0) ? bl : base));
-    }
-    const int xm = x > 0 ? x - 1 : 0, xp = x + 1 < ld ? x + 1 : x;  // edge lanes: unused
-    Cons<T, 1> a, b, fa, fb;
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      const T d = ch * limited_slope<T>(LIM, u.v[c] - src[c * ld + xm], src[c * ld + xp] - u.v[c]);
-      a.v[c] = u.v[c] - d;
-      b.v[c] = u.v[c] + d;
-    }
-    flux_q(a, derive(a, gm1), 0, fa);
-    flux_q(b, derive(b, gm1), 0, fb);
-    const T hd = T(0.5) * dtdh;
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      const T df = fa.v[c] - fb.v[c];
-      er.v[c] = b.v[c] + hd * df;
-      el.v[c] = a.v[c] + hd * df;
-    }
-  } else {
-    er = u;
-    el = u;
-  }
-  Cons<T, 1> ul, f;
-#pragma unroll
-  for (int c = 0; c < NC; ++c) ul.v[c] = up(er.v[c], 1);
-  riemann_qh<FLUX>(ul, derive(ul, gm1), el, derive(el, gm1), 0, gamma, gm1, adi, dtdh, dhdt, f,
-                   pinf);
-#pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    const T fr = dn(f.v[c], 1);
-    u.v[c] = u.v[c] + dtdh * (f.v[c] - fr);
-  }
-  return u;
 }
 
 template <typename T, int FLUX>
@@ -172,7 +115,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1)
         const int xi = x + 4 < cells + 8 ? x + 4 : cells + 7;
         const Cons<T, 1> r =
             line_cell<T, FLUX, decltype(lim)::value, decltype(muscl)::value,
-                      decltype(flat)::value>(src, ld, xi, gamma, gm1, adi, dtdh, dhdt, pinf);
+                      decltype(flat)::value, false>(src, ld, xi, gamma, gm1, adi, dtdh, dhdt, pinf);
         if (lane >= 4 && lane < 4 + kOwn && x < cells) {
           ws_max(ws, max_wavespeed_q<STIFF>(derive(r, gm1), gamma, pinf));
           // where else the cell goes: a neighbour's halo or a mirror ghost

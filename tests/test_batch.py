@@ -91,6 +91,38 @@ def test_batch_matches_oracle(cuda, oracle, dtype, mode):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("flux", ["hllc", "force"])
+def test_batch_sizes_at_the_edges(cuda, oracle, dtype, flux):
+    """1-D sizes around the 24 cells a warp updates, the size classes' bounds and
+    the smallest; 2-D sizes around the column groups with one strip and
+    several (a batch this small takes short strips)."""
+    import torch
+    from fluidity_b200.batch import Batch
+    one = np.array([[1.0, 1.0, 0.3], [0.4, 0.5, -0.2]])
+    four = np.array([[1.0, 1.0, 0.2, -0.1], [0.6, 0.5, -0.2, 0.1], [0.8, 0.7, 0.1, 0.3],
+                     [0.5, 0.9, -0.3, -0.2]])
+    probs = [((n,), one) for n in (4, 5, 23, 24, 25, 47, 48, 49, 97, 511, 512, 513, 2049)]
+    probs += [(s, four) for s in ((4, 4), (23, 9), (24, 24), (25, 31), (27, 64), (53, 130))]
+    b = Batch(probs, dtype=dtype, flux=flux)
+    b.fill()
+    steps = 8
+    b.begin(0.5, 1e30, steps)
+    b.steps(steps)
+    it, _, _, _ = b.status()
+    torch.cuda.synchronize()
+    npdt = np.float64 if dtype == "f64" else np.float32
+    for i, (shape, states) in enumerate(probs):
+        u = oracle.fill_riemann(shape, states, GAMMA, dtype=npdt)
+        ref, rit, _, _ = oracle.simulate(shape, u, npdt(GAMMA), npdt(0.5), 1.0 / shape[0],
+                                         npdt(1e30), steps, flux=flux)
+        assert it[i] == rit == steps, (i, shape)
+        tol = 1e-10 if dtype == "f64" else 2e-4
+        floor = 1e-3 if dtype == "f64" else 1.0
+        assert rel_err(b.state(i).double().cpu().numpy(), ref, floor) < tol, (i, shape)
+
+
+@pytest.mark.gpu
 def test_batch_autotune_keeps_results(cuda, oracle):
     import torch
     from fluidity_b200.batch import Batch
