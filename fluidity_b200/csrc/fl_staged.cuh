@@ -271,12 +271,11 @@ __device__ __forceinline__ void staged_strip(const SweepParams& p, const CUtenso
   for (int i = 0; i < 5; ++i) P[i] = T(0);
 #pragma unroll
   for (int i = 0; i < 3; ++i) CHA[i] = T(1);
-  // the screen: keys of positions k-1 and k-2, and per position (bit i: k-i)
-  // whether some lane may be flattened along the sweep at the position before
-  // it or across the sweep at it; halo: the same across the sweep for the
-  // bases at the warp's two edges, for the next four evolve positions
-  uint32_t key1 = 0u, key2 = 0u, hist = 0u;
-  bool halo = false;
+  // the screen: keys of positions k-1 and k-2, and per position whether some
+  // lane may be flattened along the sweep (hist_l, bit i: position k-i-1) or
+  // across it (hist_a, bit i: position k-i; bits 16-19: at the warp's edges,
+  // from position k-3)
+  uint32_t key1 = 0u, key2 = 0u, hist_l = 0u, hist_a = 0u;
 
   T* const out = static_cast<T*>(p.out);
   const int64_t pitch = p.pitch;
@@ -327,9 +326,10 @@ __device__ __forceinline__ void staged_strip(const SweepParams& p, const CUtenso
     P[4] = q.p;
     if (flat) {
       const uint32_t key = press_key(q.p);
-      const bool steep = may_flatten<T>(key, key2) |
-                         may_flatten<T>(key, __shfl_up_sync(0xffffffffu, key, 2));
-      hist = 2u * hist + (__any_sync(0xffffffffu, steep) ? 1u : 0u);
+      const bool steep_l = may_flatten<T>(key, key2);
+      const bool steep_a = may_flatten<T>(key, __shfl_up_sync(0xffffffffu, key, 2));
+      hist_l = 2u * hist_l + (__any_sync(0xffffffffu, steep_l) ? 1u : 0u);
+      hist_a = 2u * hist_a + (__any_sync(0xffffffffu, steep_a) ? 1u : 0u);
       key2 = key1;
       key1 = key;
       if (r >= 6 && (r & 3) == 2) {
@@ -340,11 +340,11 @@ __device__ __forceinline__ void staged_strip(const SweepParams& p, const CUtenso
         const uint32_t kh = press_key(derive(load(sth, qh, eoff, false, false), gm1).p);
         const uint32_t kn = __shfl_down_sync(0xffffffffu, kh, 2);
         const bool edge = (lane & 2) == 0 && may_flatten<T>(kh, kn);
-        halo = __any_sync(0xffffffffu, edge);
+        if (__any_sync(0xffffffffu, edge)) hist_a |= 0x10000u;
       }
       // ---- flattening base along the sweep of position k - 2 -------------
       // (bit 4: the base that leaves the window)
-      if (hist & 0x1eu) {
+      if (hist_l & 0x1eu) {
         CHA[0] = CHA[1];
         CHA[1] = CHA[2];
         int q3, q1;
@@ -372,8 +372,8 @@ __device__ __forceinline__ void staged_strip(const SweepParams& p, const CUtenso
       int qp;
       const T* stp = stage_back(r, 2, qp);
       const Cons<T, D> up = load(stp, qp, aoff, RF && ghost_l(j + 1), RF && flip_a);
-      T ch = T(0.5);
-      if (flat && ((hist & 0xeu) != 0u || halo)) {
+      T cx = T(1), cl = T(1);
+      if (flat && (hist_a & 0xf0008u) != 0u) {
         // ---- flattening across the sweep of (lane, j) ---------------------
         const T qp = P[1];
         const T qv = derive(uj, gm1).v[1 - S];
@@ -402,12 +402,14 @@ __device__ __forceinline__ void staged_strip(const SweepParams& p, const CUtenso
         const bool upw = sx > 0;
         const T cn = (T)chi_base<T>(upw ? pr2 : qp, upw ? qp : pl2, upw ? p3 : pr1,
                                     upw ? pl1 : p3, upw ? qv : v2, upw ? v2 : qv);
-        const T cx = std_min(chx, sx != 0 ? cn : chx);
+        cx = std_min(chi_init, std_min(chx, sx != 0 ? cn : chx));
+      }
+      if (flat && (hist_l & 0xeu) != 0u) {
         const T dl = P[2] - P[0];
         const int sl = (T(0) < dl) - (dl < T(0));
-        const T cl = std_min(CHA[1], sl > 0 ? CHA[2] : (sl < 0 ? CHA[0] : CHA[1]));
-        ch = std_min(std_min(chi_init, cx), cl) * T(0.5);
+        cl = std_min(CHA[1], sl > 0 ? CHA[2] : (sl < 0 ? CHA[0] : CHA[1]));
       }
+      const T ch = std_min(cx, cl) * T(0.5);
       Cons<T, D> a, b;
 #pragma unroll
       for (int c = 0; c < NC; ++c) {

@@ -106,10 +106,10 @@ __device__ __forceinline__ void walk_strip_2d(const SweepParams& p, T dtdh, int6
     T P[5];
     T CHY[3] = {T(1), T(1), T(1)};  // chi_y of rows k-4, k-3, k-2
     Cons<T, D> er_prev, f_prev;
-    // the flattening's screen: keys of rows k-1 and k-2, and per row (bit i:
-    // row k-i) whether some lane may be flattened along y in the row before
-    // it or along x in it
-    uint32_t key1 = 0u, key2 = 0u, hist = 0u;
+    // the flattening's screen: keys of rows k-1 and k-2, and per row whether
+    // some lane may be flattened along y (hist_y, bit i: row k-i-1) or along x
+    // (hist_x, bit i: row k-i)
+    uint32_t key1 = 0u, key2 = 0u, hist_y = 0u, hist_x = 0u;
     const int64_t k_first = y0 - 3 - (S == 1 ? 1 : 0);
     const int64_t k_last = y_end + (S == 1 ? 3 : 2);
     // row k + 1 is loaded while row k is processed (global-load latency
@@ -155,13 +155,15 @@ __device__ __forceinline__ void walk_strip_2d(const SweepParams& p, T dtdh, int6
       }
       if (flat) {
         const uint32_t key = press_key(P[4]);
-        const bool steep = may_flatten<T>(key, key2) | may_flatten<T>(key, shfl_up(key, 2));
-        hist = 2u * hist + (__any_sync(0xffffffffu, steep) ? 1u : 0u);
+        const bool steep_y = may_flatten<T>(key, key2);
+        const bool steep_x = may_flatten<T>(key, shfl_up(key, 2));
+        hist_y = 2u * hist_y + (__any_sync(0xffffffffu, steep_y) ? 1u : 0u);
+        hist_x = 2u * hist_x + (__any_sync(0xffffffffu, steep_x) ? 1u : 0u);
         key2 = key1;
         key1 = key;
         // ---- y flattening base of row k - 2 (needs rows k-4..k; bit 4: the
         // base that leaves the window) ------------------------------------
-        if (hist & 0x1eu) {
+        if (hist_y & 0x1eu) {
           CHY[0] = CHY[1];
           CHY[1] = CHY[2];
           CHY[2] = (T)chi_base<T>(P[3], P[1], P[4], P[0], U[1].v[3] * fl_rcp<T>(U[1].v[0]),
@@ -179,8 +181,8 @@ __device__ __forceinline__ void walk_strip_2d(const SweepParams& p, T dtdh, int6
         er = u;
         el = u;
       } else {
-        T ch = T(0.5);
-        if (flat && (hist & 0xeu) != 0u) {
+        T cx = T(1), cy = T(1);
+        if (flat && (hist_x & 8u) != 0u) {
           // ---- x flattening base of row j on this lane --------------------
           const T pj = P[1], vxj = u.v[2] * fl_rcp<T>(u.v[0]);
           const T p_r1 = shfl_dn(pj, 1), p_l1 = shfl_up(pj, 1);
@@ -190,12 +192,14 @@ __device__ __forceinline__ void walk_strip_2d(const SweepParams& p, T dtdh, int6
           const T chx_r = shfl_dn(chx, 1), chx_l = shfl_up(chx, 1);
           const T dx = p_r1 - p_l1;
           const int sx = (T(0) < dx) - (dx < T(0));
-          const T cx = std_min(chx, sx > 0 ? chx_r : (sx < 0 ? chx_l : chx));
+          cx = std_min(chi_init, std_min(chx, sx > 0 ? chx_r : (sx < 0 ? chx_l : chx)));
+        }
+        if (flat && (hist_y & 0xeu) != 0u) {
           const T dy = P[2] - P[0];
           const int sy = (T(0) < dy) - (dy < T(0));
-          const T cy = std_min(CHY[1], sy > 0 ? CHY[2] : (sy < 0 ? CHY[0] : CHY[1]));
-          ch = std_min(std_min(chi_init, cx), cy) * T(0.5);
+          cy = std_min(CHY[1], sy > 0 ? CHY[2] : (sy < 0 ? CHY[0] : CHY[1]));
         }
+        const T ch = std_min(cx, cy) * T(0.5);
         Cons<T, D> a, b;
 #pragma unroll
         for (int c = 0; c < NC; ++c) {

@@ -94,10 +94,10 @@ __device__ __forceinline__ void walk_strip_3d(const SweepParams& p, const T* __r
   Cons<T, D> U[5];
   T P[5];
   T CHY[3] = {T(1), T(1), T(1)};  // row-direction chi bases of rows k-4, k-3, k-2
-  // the flattening's screen: keys of rows k-1 and k-2, and per row (bit i: row
-  // k-i) whether some lane may be flattened along the rows in the row before
-  // it or along x in it
-  uint32_t key1 = 0u, key2 = 0u, hist = 0u;
+  // the flattening's screen: keys of rows k-1 and k-2, and per row whether
+  // some lane may be flattened along the rows (hist_r, bit i: row k-i-1) or
+  // along x (hist_x, bit i: row k-i)
+  uint32_t key1 = 0u, key2 = 0u, hist_r = 0u, hist_x = 0u;
   Cons<T, D> er_prev, f_prev;
   const int64_t k_first = y0 - 3 - SW;
   const int64_t k_last = y_end + 2 + SW;
@@ -151,12 +151,14 @@ __device__ __forceinline__ void walk_strip_3d(const SweepParams& p, const T* __r
     }
     if (flat) {
       const uint32_t key = press_key(P[4]);
-      const bool steep = may_flatten<T>(key, key2) | may_flatten<T>(key, shfl_up(key, 2));
-      hist = 2u * hist + (__any_sync(0xffffffffu, steep) ? 1u : 0u);
+      const bool steep_r = may_flatten<T>(key, key2);
+      const bool steep_x = may_flatten<T>(key, shfl_up(key, 2));
+      hist_r = 2u * hist_r + (__any_sync(0xffffffffu, steep_r) ? 1u : 0u);
+      hist_x = 2u * hist_x + (__any_sync(0xffffffffu, steep_x) ? 1u : 0u);
       key2 = key1;
       key1 = key;
       // the base of row k - 2 (bit 4: the base that leaves the window)
-      if (hist & 0x1eu) {
+      if (hist_r & 0x1eu) {
         CHY[0] = CHY[1];
         CHY[1] = CHY[2];
         CHY[2] = (T)chi_base<T>(P[3], P[1], P[4], P[0], U[1].v[2 + DR] * fl_rcp<T>(U[1].v[0]),
@@ -176,7 +178,7 @@ __device__ __forceinline__ void walk_strip_3d(const SweepParams& p, const T* __r
       T ch = T(0.5);
       if (flat) {
         T cx = T(1), cr = T(1);
-        if ((hist & 0xeu) != 0u) {
+        if ((hist_x & 8u) != 0u) {
           // ---- x flattening base of row j on this lane --------------------
           const T pj = P[1], vxj = u.v[2] * fl_rcp<T>(u.v[0]);
           const T p_r1 = shfl_dn(pj, 1), p_l1 = shfl_up(pj, 1);
@@ -187,6 +189,8 @@ __device__ __forceinline__ void walk_strip_3d(const SweepParams& p, const T* __r
           const T dx = p_r1 - p_l1;
           const int sx = (T(0) < dx) - (dx < T(0));
           cx = std_min(chi_init, std_min(chx, sx > 0 ? chx_r : (sx < 0 ? chx_l : chx)));
+        }
+        if ((hist_r & 0xeu) != 0u) {
           const T dy = P[2] - P[0];
           const int sy = (T(0) < dy) - (dy < T(0));
           cr = std_min(CHY[1], sy > 0 ? CHY[2] : (sy < 0 ? CHY[0] : CHY[1]));
