@@ -182,6 +182,28 @@ def test_ghost_matches_oracle(cuda, oracle, dtype, seed):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny", [(29, 40), (30, 8), (31, 9), (61, 33), (92, 17)])
+def test_ghost_at_scan_edges(cuda, oracle, nx, ny):
+    """An interface that crosses the grid aslant, so that sources, their targets
+    and the band lie on either side of the scan's column groups (30 wide), of
+    its strips (8 rows) and of the domain's ends: bit for bit the oracle's."""
+    spec = _spec(seed=6, nx=nx, ny=ny)
+    h = spec["h"]
+    X, Y = np.meshgrid(np.arange(nx) + 0.5, np.arange(ny) + 0.5)
+    line = ((X - 0.5 * nx) * 0.8 * min(1.0, ny / nx) + (Y - 0.5 * ny)) * h
+    spec["phi0"] = (line / np.hypot(0.8 * min(1.0, ny / nx), 1.0)).reshape(-1)
+    spec["phi1"] = -spec["phi0"]
+    u0, u1 = _initial(spec, perturb=1.0, seed=6)
+    w0, w1 = oracle.mm_ghost(nx, ny, h, spec["gammas"], u0, u1, spec["phi0"], spec["phi1"])
+    mm = _device_mm(spec, "f64", u0, u1)
+    mm.ghost()
+    st = mm.stats()
+    assert st["gfm0"] > 0 and st["gfm1"] > 0 and st["band0"] > 0 and st["band1"] > 0
+    g0, g1 = (t.cpu().numpy() for t in mm.states())
+    assert np.array_equal(g0, w0) and np.array_equal(g1, w1)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype", ["f64", "f32"])
 def test_steps_match_oracle(cuda, oracle, dtype):
     spec = _spec(seed=4, nx=96, ny=48)
