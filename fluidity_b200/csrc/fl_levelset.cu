@@ -46,25 +46,21 @@ __device__ __forceinline__ int64_t lmir(int64_t i, int64_t n) {
 
 __device__ __forceinline__ double dmin_(double a, double b) { return (b < a) ? b : a; }
 
-// One thread per cell: x from blockIdx.x, rows from blockIdx.y (strided when
-// the grid has more rows than a launch's y extent), which spares the 64-bit
-// division that splits the index of a grid-stride loop.
 template <typename T>
-__global__ void __launch_bounds__(256)
-    ls_velocity_kernel(int64_t nx, int64_t ny, int nmat, const double* phi0, const double* phi1,
-                       const T* u0, const T* u1, int64_t pitch, double h, double* vel) {
-  const int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= nx) return;
-  const double fact = 0.5 / h;
-  const int64_t xm = lmir(x - 1, nx), xp = lmir(x + 1, nx);
-  for (int64_t y = blockIdx.y; y < ny; y += gridDim.y) {
-    const int64_t i = y * nx + x;
+__global__ void ls_velocity_kernel(int64_t nx, int64_t ny, int nmat, const double* phi0,
+                                   const double* phi1, const T* u0, const T* u1, int64_t pitch,
+                                   double h, double* vel) {
+  const int64_t n = nx * ny;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t x = i % nx, y = i / nx;
     double v = 0.0;
     for (int m = 0; m < nmat; ++m) {
       const double* f = m == 0 ? phi0 : phi1;
       const T* u = m == 0 ? u0 : u1;
       if (!(f[i] <= 0.0 || f[i] <= -0.0)) continue;
-      const double g0 = fact * (f[y * nx + xp] - f[y * nx + xm]);
+      const double fact = 0.5 / h;
+      const double g0 = fact * (f[y * nx + lmir(x + 1, nx)] - f[y * nx + lmir(x - 1, nx)]);
       const double g1 = fact * (f[lmir(y + 1, ny) * nx + x] - f[lmir(y - 1, ny) * nx + x]);
       const double s = sqrt(g0 * g0 + g1 * g1);
       const double rho = (double)u[i];
@@ -350,19 +346,18 @@ int fl_ls_velocity(const fl_grid* grid, int nmat, const double* const* phis,
     if (!phis[m] || !states[m]) return set_error(kEInval, "NULL material %d", m);
   if (pitch < grid->n[0] * grid->n[1]) return set_error(kEInval, "pitch below the cell count");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int64_t n = grid->n[0] * grid->n[1];
   const double* p1 = nmat > 1 ? phis[1] : phis[0];
-  const dim3 vg((unsigned)((grid->n[0] + 255) / 256),
-                (unsigned)(grid->n[1] < 65535 ? grid->n[1] : 65535));
   if (policy & 1u) {
     const float* u1 = static_cast<const float*>(nmat > 1 ? states[1] : states[0]);
-    ls_velocity_kernel<float><<<vg, 256, 0, st>>>(grid->n[0], grid->n[1], nmat, phis[0], p1,
-                                                  static_cast<const float*>(states[0]), u1, pitch,
-                                                  h, vel);
+    ls_velocity_kernel<float><<<grid1d(n), 256, 0, st>>>(grid->n[0], grid->n[1], nmat, phis[0], p1,
+                                                         static_cast<const float*>(states[0]), u1,
+                                                         pitch, h, vel);
   } else {
     const double* u1 = static_cast<const double*>(nmat > 1 ? states[1] : states[0]);
-    ls_velocity_kernel<double><<<vg, 256, 0, st>>>(grid->n[0], grid->n[1], nmat, phis[0], p1,
-                                                   static_cast<const double*>(states[0]), u1,
-                                                   pitch, h, vel);
+    ls_velocity_kernel<double><<<grid1d(n), 256, 0, st>>>(grid->n[0], grid->n[1], nmat, phis[0],
+                                                          p1, static_cast<const double*>(states[0]),
+                                                          u1, pitch, h, vel);
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error(kECuda, "fl_ls_velocity: %s", cudaGetErrorString(e));
