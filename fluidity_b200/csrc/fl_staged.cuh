@@ -291,6 +291,11 @@ __device__ __forceinline__ void staged_strip(const SweepParams& p, const CUtenso
   constexpr bool RF = !FAST;
   const bool flat = FAST || flatten;
   const bool mus = FAST || muscl;
+  // the common form takes two positions per turn: the windows' moves and the
+  // loop's own tests fall by half (4096^2 FP64 HLLC 1.2% faster, 1920 x 1080
+  // FP32 2.8%); four positions leave the instruction cache (11% and 4% slower)
+  constexpr int kTurn = FAST ? 2 : 1;
+#pragma unroll kTurn
   for (int r = 0; r < nr; ++r) {
     const int k = k_first + r;
     // ---- ring: recycle the stage the walk no longer reads, wait for k ----
