@@ -18,8 +18,8 @@
 //    interface keep |phi| (scheme/cuda/fast_iterative_method.cuh:48-89, which
 //    seeds the signed value), every other cell
 //    relaxes to the fixed point of the Godunov local eikonal solve
-//    (schemes/godunov_upwind_scheme.hpp:44-53); 16x16 tiles relax in shared
-//    memory, passes ping-pong between two buffers, only tiles stamped by a
+//    (schemes/godunov_upwind_scheme.hpp:44-53); 32x32 tiles are swept along
+//    their diagonals in shared memory, passes ping-pong between two buffers, only tiles stamped by a
 //    changed neighbour relax in the next pass (a worklist: a changed tile
 //    and those of its 4 edge neighbours whose shared edge changed; the
 //    others hold the same values in both buffers), and the host checks

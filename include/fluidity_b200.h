@@ -473,7 +473,7 @@ int fl_ls_project(int64_t cells, double* a, double* b, void* stream);
 
 /* Reinitialisation to a signed distance (fast iterative method): cells next
  * to a sign change keep |phi|, every other cell converges to the Godunov
- * eikonal fixed point, the result takes phi's sign.  Active 16x16 tiles,
+ * eikonal fixed point, the result takes phi's sign.  Active 32x32 tiles,
  * at most max_passes passes (FL_ETIMEOUT beyond); *passes (nullable) gets
  * the count.  Replaces scheme/cuda/fast_iterative_method.cuh:48-112 and its
  * driver (fast_iterative, :366-); the reference seeds sources with the signed

@@ -9,7 +9,7 @@ contraction and use IEEE division and square root, so they match the oracle
 bit for bit.  The RK3 advection contracts into FMAs and normalises the WENO
 weights with one reciprocal per derivative; it agrees with the oracle to
 1e-12 of max |phi|, one step or twenty.  The reinitialisation relaxes in a
-different order (16x16 tiles against whole-grid Jacobi sweeps); its fixed
+different order (32x32 tiles against whole-grid Jacobi sweeps); its fixed
 point agrees to 1e-12 of max |phi|.
 """
 import numpy as np
